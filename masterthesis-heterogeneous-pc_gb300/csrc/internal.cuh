@@ -322,7 +322,7 @@ hpc_status launch_standardise(const void *X, bool f32, const StdArgs &a, long lo
 hpc_status launch_pair_to_f64(const float *zh, const float *zl, long long count, double *Z, cudaStream_t s);
 struct GramArgs {                   // grouped FP64 Gram
   int count;
-  const long long *tile_prefix;     // 64 x 64 upper-triangle tiles (count + 1)
+  const long long *tile_prefix;     // gram_f64_tiles(p) per instance (count + 1)
   const long long *z_off, *c_off, *n, *p;
   const double *denom;
 };
