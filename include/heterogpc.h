@@ -124,7 +124,9 @@ hpc_status hpc_ctx_set_stream(hpc_ctx *ctx, void *stream);
 hpc_status hpc_ctx_set_graphs(hpc_ctx *ctx, int enable);
 /* Device-time breakdown of the context's last correlation and levels. */
 hpc_status hpc_get_timings(hpc_ctx *ctx, hpc_timings *out);
-/* Device bytes held by a context of this shape (admission control). */
+/* Device bytes held by a context of this shape (admission control). Dense graphs take more,
+ * as they come: neighbour lists and records for their edges, and up to about 6 MB a thread block
+ * (two blocks an SM) for levels 1 and 2 on wide rows, which run without where there is no room. */
 hpc_status hpc_ctx_footprint(int64_t p, int64_t n_obs, const hpc_opts *opts, int64_t *bytes);
 
 /* ---- correlation --------------------------------------------------------
@@ -376,6 +378,10 @@ hpc_status hpc_debug_set_order_from(int level);
  * the context (1 while the set order is in use). */
 hpc_status hpc_debug_set_retest_queue(hpc_ctx *ctx, int64_t entries);
 int hpc_debug_set_order_active(hpc_ctx *ctx);
+/* hpc_debug_set_wide(ctx, level1, level2): whether levels 1 and 2 of the context's runs use
+ * the kernels for wide rows (mixed precision): 1 yes, 0 no, -1 the library's rules (the
+ * default). Every choice gives the same skeleton. */
+hpc_status hpc_debug_set_wide(hpc_ctx *ctx, int level1, int level2);
 
 /* ---- synthetic data ------------------------------------------------------
  * Seeded linear-Gaussian SEM (no reference counterpart; the reference reads

@@ -1,9 +1,9 @@
 // Level-l CI tests (l >= 1): the re-test and record kernels, the level-kernel
 // instantiations of levels 1-8 and the launchers (the level kernels' device code is in
-// citest.cuh).
+// citest.cuh, wide.cuh and level_kernel.cuh).
 #include <algorithm>
 
-#include "citest.cuh"
+#include "level_kernel.cuh"
 
 namespace hpc {
 namespace {
@@ -427,12 +427,19 @@ void *kernel_for(int level, int l1_variant) {
   }
   switch (level) {
     case 1:
+      if constexpr (MIXED) {
+        if (l1_variant == kWide) return (void *)level_kernel<1, true, kWide>;
+        if (l1_variant == (kWide | kQueueOnly)) return (void *)level_kernel<1, true, kWide | kQueueOnly>;
+      }
       if (MIXED && l1_variant == (kL1Interleaved | kQueueOnly)) return (void *)level_kernel<1, true, kL1Interleaved | kQueueOnly>;
       if (MIXED && l1_variant == (kL1Prefetch | kQueueOnly)) return (void *)level_kernel<1, true, kL1Prefetch | kQueueOnly>;
       return l1_variant == kL1Chunked    ? (void *)level_kernel<1, MIXED, kL1Chunked>
              : l1_variant == kL1Prefetch ? (void *)level_kernel<1, MIXED, kL1Prefetch>
                                          : (void *)level_kernel<1, MIXED>;
-    case 2: return (void *)level_kernel<2, MIXED>;
+    case 2:
+      if constexpr (MIXED)
+        if (l1_variant == kWide) return (void *)level_kernel<2, true, kWide>;
+      return (void *)level_kernel<2, MIXED>;
     case 3: return (void *)level_kernel<3, MIXED>;
     case 4: return (void *)level_kernel<4, MIXED>;
     case 5: return (void *)level_kernel<5, MIXED>;
@@ -445,12 +452,19 @@ void *kernel_for(int level, int l1_variant) {
   }
 }
 
+// dynamic shared memory of a level kernel: the row-offset cache of levels >= 2, the chunk of
+// the wide level-1 body
+int level_smem(int level, int variant) {
+  if (level == 1) return (variant & kWide) ? (int)sizeof(Wide1Smem) : 0;
+  return kRowCache * (int)sizeof(unsigned long long);
+}
+
 }  // namespace
 
 int citest_grid(int precision, int level, int device, int l1_variant) {
   void *k = precision == HPC_PREC_FP64 ? kernel_for<false>(level, l1_variant) : kernel_for<true>(level, l1_variant);
-  const int smem = level == 1 ? 0 : kRowCache * (int)sizeof(unsigned long long);
-  // the row-offset cache is beyond the default 48 KB of dynamic shared memory
+  const int smem = level_smem(level, l1_variant);
+  // beyond the default 48 KB of shared memory
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) cudaGetLastError();
   int per_sm = 0, sms = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem) != cudaSuccess || per_sm < 1)
@@ -514,7 +528,7 @@ hpc_status launch_level(const Launch &L, int precision, int grid, int l1_variant
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = L.level == 1 || !L.row_cache ? 0 : kRowCache * sizeof(unsigned long long);
+  cfg.dynamicSmemBytes = L.level > 1 && !L.row_cache ? 0 : (size_t)level_smem(L.level, l1_variant);
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;

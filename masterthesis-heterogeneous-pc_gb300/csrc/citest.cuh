@@ -658,12 +658,12 @@ __device__ __forceinline__ void skip_tiles_of_edge(const Launch &L, unsigned lon
 // (mixed precision: levels 2-16 of the edge order, every set-order level) the staged
 // correlation block.
 template <int LT, bool MIXED>
-struct TestSmem {
+struct alignas(16) TestSmem {
   static constexpr int LA = LT > 0 ? LT : HPC_MAX_LEVEL;
   static constexpr bool kBlk = MIXED && LT >= 2 && LT <= kSetTop;
   PendRem<LA> pend[kThreads / 32][kPend];
   int np[kThreads / 32];
-  float blk[kBlk ? kThreads / 32 : 1][kBlk ? kBlkS * kBlkS : 1];
+  alignas(16) float blk[kBlk ? kThreads / 32 : 1][kBlk ? kBlkS * kBlkS : 1];
 };
 
 template <int LT, bool MIXED>
@@ -1409,39 +1409,6 @@ __device__ __forceinline__ void tests_set(const Launch &L, unsigned long long *r
       if (rt) atomicAdd(&inst_of(L, b_last)->ctr[level].retests, (unsigned long long)rt);
     }
   }
-}
-
-// One level l >= 1: rebuild | grid barrier | scan | grid barrier | CI tests. LT = 1
-// is the lane-interleaved level-1 body (V: kL1Prefetch loads one step ahead,
-// kL1Chunked runs the chunked body of the higher levels; picked by the tile policy),
-// LT = 2..16 the bodies unrolled for l = LT (V = kSetOrder: in the set order, LT up to
-// kSetTop), LT = 0 the runtime-level body.
-template <int LT, bool MIXED, int V = kL1Interleaved>
-__global__ void __launch_bounds__(kThreads, V == kSetOrder ? kSetBlocks<LT> : (LT == 1 && (V & 3) != kL1Chunked ? 4 : 2))
-    level_kernel(const __grid_constant__ Launch L) {
-  extern __shared__ unsigned long long rw_smem[];  // kRowCache entries
-  unsigned int epoch = 0;
-  const bool stamp = blockIdx.x == 0 && threadIdx.x == 0;  // the phase times
-  if (stamp) L.lc->t_entry = globaltimer_ns();
-  rebuild_phase(L);
-  if (!grid_barrier(L, epoch)) return;
-  if (stamp) L.lc->t_rebuilt = globaltimer_ns();
-  scan_phase(L, V == kSetOrder);
-  if (!grid_barrier(L, epoch)) return;
-  if (stamp) L.lc->t_scanned = globaltimer_ns();
-  const TuneEntry te = tile_policy(L);
-  if constexpr (V == kSetOrder) {
-    static_assert(MIXED && LT >= 2 && LT <= kSetTop, "the set order runs levels 2-24 in mixed precision");
-    __shared__ TestSmem<LT, true> sm;
-    tests_set<LT>(L, rw_smem, te, sm);
-  } else if constexpr (LT == 1 && (V & 3) != kL1Chunked) {  // level 1 keeps the SM's on-chip memory for L1 cache
-    tests_l1<MIXED, (V & 3) == kL1Prefetch, (V & kQueueOnly) != 0>(L, nullptr, te);
-  } else {
-    __shared__ TestSmem<LT, MIXED> sm;
-    tests_generic<LT, MIXED>(L, LT == 1 ? nullptr : rw_smem, te, sm);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) atomicMax(&L.lc->t_end, globaltimer_ns());
 }
 
 }  // namespace

@@ -1,6 +1,6 @@
 // Level kernels of levels 13-16 (a translation unit of their own, so that the
 // level instantiations compile in parallel).
-#include "citest.cuh"
+#include "level_kernel.cuh"
 
 namespace hpc {
 

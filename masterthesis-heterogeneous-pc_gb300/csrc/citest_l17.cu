@@ -3,7 +3,7 @@
 // unrolled). Levels this high are reached only by graphs whose neighbour lists stay
 // long (skeletons run until no edge has enough neighbours); a translation unit of its
 // own so that it compiles in parallel with the unrolled levels.
-#include "citest.cuh"
+#include "level_kernel.cuh"
 
 namespace hpc {
 

@@ -3,7 +3,7 @@
 // neighbours, where the runtime-level kernel of citest_l17.cu (arrays sized for 32
 // members, loops not unrolled) spends most of its time in local memory. A translation
 // unit of its own so that it compiles in parallel with the other levels.
-#include "citest.cuh"
+#include "level_kernel.cuh"
 
 namespace hpc {
 

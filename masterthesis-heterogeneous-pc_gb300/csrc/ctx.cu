@@ -187,6 +187,7 @@ hpc_status write_inst_table(hpc_ctx *c) {
     I.n_z = h.n;
     I.denom = denom_of(c, h.n);
     I.adj = c->adj + h.adj_off;
+    I.adj0 = c->adj0 ? c->adj0 + h.adj_off : nullptr;
     I.deg = c->deg + h.row_off;
     I.rowptr = c->rowptr + h.row_off;
     I.row_work = c->row_work + h.row_off;
@@ -267,6 +268,12 @@ Launch make_launch(hpc_ctx *c, int level) {
   L.inst0 = c->inst_host[0];
   L.wait_ns = c->wait_ns;
   L.bar_extra = c->bar_extra;
+  L.p_max = c->p_max;
+  L.wide_cols = c->wide_cols;
+  L.wide_items = c->wide_items;
+  L.wide_cap = (unsigned int)c->wide_cap;
+  L.wide_scratch = c->wide_scratch;
+  L.wide_floats = c->wide_floats;
   return L;
 }
 
@@ -305,11 +312,14 @@ hpc_status enqueue_level(hpc_ctx *c, int level, bool timed) {
   const bool set = set_at(c, level);
   // level 1: the queue-only build of the interleaved variants where the re-tests are
   // queued and a queue overflow can be rerun
-  const bool qo = level == 1 && c->l1v_now != kL1Chunked && effective_set_from(c) > 0;
-  const int var = level == 1 ? (qo ? c->l1v_now | kQueueOnly : c->l1v_now) : set ? kSetOrder : kL1Interleaved;
-  const int grid = level == 1 ? (qo ? c->citest_grid_l1q[c->l1v_now] : c->citest_grid_l1[var])
-                   : set      ? c->citest_grid_set[level]
-                              : c->citest_grid[level];
+  const bool wide = (level == 1 && c->wide1) || (level == 2 && c->wide2 && !set);
+  const bool qo = level == 1 && (wide || c->l1v_now != kL1Chunked) && effective_set_from(c) > 0;
+  const int l1v = wide ? kWide : c->l1v_now;
+  const int var = level == 1 ? (qo ? l1v | kQueueOnly : l1v) : set ? kSetOrder : wide ? kWide : kL1Interleaved;
+  const int grid = wide         ? c->citest_grid_wide[level == 2 ? 2 : qo ? 1 : 0]
+                   : level == 1 ? (qo ? c->citest_grid_l1q[c->l1v_now] : c->citest_grid_l1[var])
+                   : set        ? c->citest_grid_set[level]
+                                : c->citest_grid[level];
   if ((s = launch_level(L, c->opts.precision, grid, var, c->stream)) != HPC_OK) return s;
   if (timed) HPC_CUDA(cudaEventRecord(ev[3], c->stream));
   if (queue && (s = launch_retest(L, c->sm_count, c->stream)) != HPC_OK) return s;
@@ -509,6 +519,52 @@ hpc_status sync_tune(hpc_ctx *c) {
   return HPC_OK;
 }
 
+// Which of levels 1 and 2 run the wide-row kernels (wide.cuh) in the runs being queued, and
+// their buffers: level 1 by the rule on the level-0 result of the context's data (or of its last
+// run), level 2 where rows were much wider than kWideDeg in the last run -- before a first run,
+// where level 1 is wide. (The kernel of level 2 takes the wide rows and leaves the others to the
+// ordinary body, so a wrong guess costs time only.) Without room for the buffers the ordinary
+// kernels run.
+hpc_status choose_wide(hpc_ctx *c) {
+  c->wide1 = c->wide2 = false;
+  if (c->opts.precision == HPC_PREC_FP64) return HPC_OK;
+  const bool forced_policy = c->tune_force.tile_cap > 0 && !c->tuning;  // a forced policy picks its kernels
+  std::vector<WideShape> sh((size_t)c->count);
+  for (int b = 0; b < c->count; ++b)
+    sh[b] = WideShape{c->ih[b].p, c->level0_known ? (int64_t)c->ctr_host[(size_t)b * kLevels].edges2 : 0};
+  if (c->level0_known && !forced_policy && !c->wide_denied) {
+    c->wide1 = wide1_pays(sh.data(), c->count);
+    c->wide2 = c->deg_seen[2] >= 0 ? c->deg_seen[2] >= 4 * kWideDeg : c->wide1;
+  }
+  if (c->wide_force1 >= 0) c->wide1 = c->wide_force1 > 0;
+  if (c->wide_force2 >= 0) c->wide2 = c->wide_force2 > 0;
+  hpc_status s = HPC_OK;
+  if (c->wide1) {
+    const int cols = wide1_cols(sh.data(), c->count);
+    if (cols != c->wide_cols) ++c->inst_version;  // a launch parameter
+    c->wide_cols = cols;
+    if (!c->adj0) {
+      s = dev_alloc(&c->adj0, c->total_words, "adjacency snapshot");
+      if (s == HPC_OK && (s = write_inst_table(c)) != HPC_OK) return s;
+    }
+  }
+  if (c->wide2 && !c->wide_scratch && s == HPC_OK) {
+    long long cap = 0;
+    for (const auto &h : c->ih) cap += h.p * wide2_slices(h.p - 1, h.p);
+    if (!c->wide_items) s = dev_alloc(&c->wide_items, cap, "wide-row queue");
+    c->wide_cap = cap;
+    c->wide_floats = wide2_floats(c->p_max - 1);
+    if (s == HPC_OK) s = dev_alloc(&c->wide_scratch, c->wide_floats * c->citest_grid_wide[2], "wide-row scratch");
+    if (s == HPC_OK) ++c->inst_version;  // a captured graph holds no pointers to them
+  }
+  if (s != HPC_OK) {
+    c->wide1 = c->wide1 && c->adj0;
+    c->wide2 = c->wide2 && c->wide_scratch;
+    c->wide_denied = true;
+  }
+  return HPC_OK;
+}
+
 // Run levels first..last with one host sync at the end; the whole sequence 0..last
 // is captured once into a CUDA graph and replayed while the buffers stay in place.
 // `finalize` appends the FP64 p-values of the FP32-decided removals (and their FP64
@@ -519,6 +575,7 @@ hpc_status run_levels(hpc_ctx *c, int first, int last, bool use_graph, bool wait
   hpc_status s;
   if ((s = sync_tune(c)) != HPC_OK) return s;
   c->l1v_now = level1_variant(c);
+  if (last >= 1 && (s = choose_wide(c)) != HPC_OK) return s;
   finalize = finalize && last >= 1 && c->recs;
   auto enqueue_all = [&](bool timed) -> hpc_status {
     if (first == 0) {  // a skeleton from the start: its counters and records begin at zero
@@ -539,7 +596,8 @@ hpc_status run_levels(hpc_ctx *c, int first, int last, bool use_graph, bool wait
   if (last >= 1) c->records_final = finalize;
   if (use_graph && c->graphs_enabled && first == 0 && capturable(c->stream)) {
     const bool valid = c->graph && c->graph_top == last && c->graph_stream == c->stream &&
-                       c->graph_version == c->inst_version && c->graph_l1v == c->l1v_now &&
+                       c->graph_version == c->inst_version && c->graph_l1v == (c->wide1 ? kWide : c->l1v_now) &&
+                       c->graph_wide2 == c->wide2 &&
                        c->graph_set_mask == set_mask(c, last) &&
                        c->graph_final == finalize;
     if (!valid) {
@@ -565,7 +623,8 @@ hpc_status run_levels(hpc_ctx *c, int first, int last, bool use_graph, bool wait
       c->graph_top = last;
       c->graph_stream = c->stream;
       c->graph_version = c->inst_version;
-      c->graph_l1v = c->l1v_now;
+      c->graph_l1v = c->wide1 ? kWide : c->l1v_now;
+      c->graph_wide2 = c->wide2;
       c->graph_set_mask = set_mask(c, last);
       c->graph_final = finalize;
     }
@@ -576,7 +635,10 @@ hpc_status run_levels(hpc_ctx *c, int first, int last, bool use_graph, bool wait
     if ((s = enqueue_all(true)) != HPC_OK) return s;
     c->last_run_graph = false;
   }
-  return wait ? pull_counters(c) : HPC_OK;
+  if (!wait) return HPC_OK;
+  if ((s = pull_counters(c)) != HPC_OK) return s;
+  c->level0_known = true;
+  return HPC_OK;
 }
 
 // ---- correlation ----------------------------------------------------------
@@ -860,6 +922,34 @@ bool uses_set_order(int set_from, int level) {
   return set_from > 0 && level >= 2 && level <= kSetTop && level >= set_from;
 }
 
+// Level 1 on wide rows costs a filter step for every variable and pair i < j (sum over the
+// instances of edges2 / 2 * p), the ordinary level-1 body many times that for every potential
+// test (about edges2^2 / p): the wide body where the latter come to kWide1Ratio of the former
+// or more, that is above a mean degree of p / 16, and where there are items for every SM.
+constexpr double kWide1Ratio = 1.0 / 8.0;
+static double wide1_items(const WideShape *sh, int count, int cols) {
+  double t = 0.0;
+  for (int b = 0; b < count; ++b)
+    t += (double)((sh[b].p + kW1Rows - 1) / kW1Rows) * (double)((sh[b].p + cols - 1) / cols) * 0.5;
+  return t;
+}
+bool wide1_pays(const WideShape *sh, int count) {
+  double filter = 0.0, tests = 0.0;
+  for (int b = 0; b < count; ++b) {
+    const double e2 = (double)sh[b].edges2, p = (double)sh[b].p;
+    filter += 0.5 * e2 * p;
+    tests += e2 * e2 / p;
+  }
+  return tests > kWide1Ratio * filter && wide1_items(sh, count, 256) >= 152.0;
+}
+// as many columns as leave eight items for every SM (an item's rows are copied once for all of
+// them), 256 (a 32-column word for each warp) at least
+int wide1_cols(const WideShape *sh, int count) {
+  int cols = 1024;
+  while (cols > 256 && wide1_items(sh, count, cols) < 8 * 152.0) cols /= 2;
+  return cols;
+}
+
 // for the server's shared launches (serve.cu)
 hpc_status ctx_size_after_level0(hpc_ctx *c) {
   bool changed = false;
@@ -972,6 +1062,9 @@ hpc_status hpc_ctx_destroy(hpc_ctx *c) {
     c->X_stage = nullptr;
   }
   dev_free(c->adj);
+  dev_free(c->adj0);
+  dev_free(c->wide_items);
+  dev_free(c->wide_scratch);
   dev_free(c->adj_bytes);
   dev_free(c->deg);
   dev_free(c->rowptr);
@@ -1081,6 +1174,7 @@ hpc_status hpc_autotune(hpc_ctx *c, const hpc_tune_params *cands, int ncands, in
   }
   const bool graphs = c->graphs_enabled;
   const TuneEntry force0 = c->tune_force;
+  c->tuning = true;
   c->graphs_enabled = false;  // kernel by kernel: every level's kernels are timed
   // every candidate's level times, the candidates taken in turn within each round (so
   // that a drift over the tuning run touches them alike); per level the candidate with
@@ -1121,6 +1215,7 @@ hpc_status hpc_autotune(hpc_ctx *c, const hpc_tune_params *cands, int ncands, in
     }
   }
   c->tune_force = force0;
+  c->tuning = false;
   c->graphs_enabled = graphs;
   ++c->inst_version;
   const hpc_status reset = hpc_ctx_reset(c);
@@ -1788,6 +1883,19 @@ hpc_status hpc_debug_set_retest_queue(hpc_ctx *c, int64_t entries) {
   return HPC_OK;
 }
 
+hpc_status hpc_debug_set_wide(hpc_ctx *c, int level1, int level2) {
+  hpc_status s = check_ctx(c);
+  if (s != HPC_OK) return s;
+  if (level1 < -1 || level1 > 1 || level2 < -1 || level2 > 1) {
+    set_error("wide rows: -1 (the rule), 0 or 1");
+    return HPC_ERR_INVALID_ARG;
+  }
+  if ((s = settle(c)) != HPC_OK) return s;
+  c->wide_force1 = level1;
+  c->wide_force2 = c->rec_ids >= 2 ? level2 : -1;
+  return HPC_OK;
+}
+
 int hpc_debug_set_order_active(hpc_ctx *c) { return c && !c->set_off ? 1 : 0; }
 
 hpc_status hpc_debug_set_order_from(int level) {
@@ -1925,6 +2033,7 @@ hpc_status create(hpc_ctx **out, int count, const int64_t *p, const int64_t *n, 
   {
     int64_t pmax = 0;
     for (const auto &h : c->ih) pmax = std::max<int64_t>(pmax, h.p);
+    c->p_max = pmax;
     c->p_bucket = tune_bucket(pmax, kTunePB);
   }
   hpc_status s = HPC_OK;
@@ -1959,6 +2068,11 @@ hpc_status create(hpc_ctx **out, int count, const int64_t *p, const int64_t *n, 
     for (int l = 2; l <= std::min(c->rec_ids, kSetTop); ++l)
       c->citest_grid_set[l] = citest_grid(o.precision, l, c->device, kSetOrder);
   for (int v = 0; v < 3; ++v) c->citest_grid_l1[v] = citest_grid(o.precision, 1, c->device, v);
+  if (o.precision != HPC_PREC_FP64) {
+    c->citest_grid_wide[0] = citest_grid(o.precision, 1, c->device, kWide);
+    c->citest_grid_wide[1] = citest_grid(o.precision, 1, c->device, kWide | kQueueOnly);
+    if (c->rec_ids >= 2) c->citest_grid_wide[2] = citest_grid(o.precision, 2, c->device, kWide);
+  }
   if (o.precision != HPC_PREC_FP64)
     for (int v = 0; v < 2; ++v) c->citest_grid_l1q[v] = citest_grid(o.precision, 1, c->device, v | kQueueOnly);
   if (c->rec_ids > 16) retest_setup();  // the re-test kernel of levels 17-32

@@ -68,7 +68,9 @@ struct LaunchCounters {
   unsigned int scan_done;          // scan blocks finished (the last one forms the prefix)
   unsigned int bar;                // grid-barrier arrivals of the level kernel
   int max_deg;                     // largest degree at the level start over all instances
-  int pad;
+  // level 2's queue of wide rows (wide.cuh): items of the widest rows, of the others,
+  // and the next item to take
+  unsigned int wide_front, wide_back, wide_next;
   // %globaltimer (ns) of the level kernel's phases: block 0 at entry, after the rebuild
   // and after the scan; the last block to finish its tests
   unsigned long long t_entry, t_rebuilt, t_scanned, t_end;
@@ -90,6 +92,9 @@ constexpr int kL1Interleaved = 0, kL1Prefetch = 1, kL1Chunked = 2;
 // (citest.cuh) instead of the edge order (variant 0)
 constexpr int kSetOrder = 3;
 constexpr int kSetTop = 24;  // the highest level with a set-order kernel (unrolled for its level)
+// kernel variant of levels 1 and 2 for wide rows (wide.cuh): level 1 over whole rows of the
+// matrix, level 2 with the rows of kWideDeg neighbours or more on a copied block
+constexpr int kWide = 4;
 // flag on the level-1 variants kL1Interleaved / kL1Prefetch: undecided tests only
 // queued (mixed precision without an FP64 matrix), as the set order does
 constexpr int kQueueOnly = 8;
@@ -110,12 +115,47 @@ constexpr int kSegRows = 256;
 struct SegAgg {
   unsigned long long deg;   // sum of degrees
   unsigned long long work;  // sum of tests per row
-  unsigned long long sets;  // sum of conditioning sets per row (the units of the set order)
+  unsigned long long sets;  // sum of conditioning sets per row (the units of the set order), or of the
+                            // narrow rows' tests (the wide-row kernel of level 2)
   int max_deg;
   int rows;                 // rows with tests
   int over;                 // a row's test count does not fit
   int pad;
 };
+constexpr int kW1Rows = 16;  // rows of an item of the wide level-1 body (wide.cuh)
+// Level 2's wide rows (wide.cuh): rows of kWideDeg neighbours or more at the level's start;
+// an item of their queue is a row with one slice of its neighbours (every wide2_slices-th,
+// from `slice` on).
+constexpr int kWideDeg = 32, kWideFirst = 256;  // rows of kWideFirst neighbours or more go first
+struct WideItem {
+  int32_t inst, row, slice;
+};
+constexpr int kW2Slice = 1024;  // most neighbours of a slice
+constexpr int kW2Super = 32;    // rows copied at a time beside a slice that does not hold them all
+constexpr int64_t kW2Floats = 1 << 20;  // copied entries of a slice, about
+// leading dimension of the copied block of a row of degree d: the row itself and its neighbours,
+// rows of whole 16-byte words
+__host__ __device__ __forceinline__ int64_t wide2_ld(int64_t d) { return (d + 1 + 3) & ~(int64_t)3; }
+// A row is split where its slice would not fit the scratch, and below p = 6000 also at 256
+// neighbours: there are too few rows then to keep every block busy beside its widest ones
+// (p = 3001: 5.2 -> 3.0 ms), while with more rows the copies of the rows beside the slices cost
+// more than they save (p = 9000: 79 -> 48 ms without).
+__host__ __device__ __forceinline__ int wide2_slice(int64_t d, int64_t p) {
+  const int64_t s = kW2Floats / wide2_ld(d), most = p < 6000 ? 256 : kW2Slice;
+  return (int)(s < 32 ? 32 : s > most ? most : s);
+}
+__host__ __device__ __forceinline__ int wide2_slices(int64_t d, int64_t p) {
+  const int s = wide2_slice(d, p);
+  return (int)((d + s - 1) / s);
+}
+// scratch floats of a block that serves rows of up to d neighbours: row i, a slice, the rows
+// beside it (the slice holds at most kW2Floats entries, or 32 rows)
+inline int64_t wide2_floats(int64_t d) {
+  const int64_t ld = wide2_ld(d), all = (d < kW2Slice ? d : kW2Slice) * ld;
+  const int64_t most = kW2Floats > 32 * ld ? kW2Floats : 32 * ld;
+  return (1 + kW2Super) * ld + (all < most ? all : most);
+}
+
 constexpr int kErrRecOverflow = 1;
 constexpr int kErrWorkOverflow = 2;
 constexpr int kErrCsrOverflow = 4;
@@ -164,6 +204,7 @@ struct Inst {
   int64_t n_z;
   double denom;           // the Gram's divisor n - 1
   uint32_t *adj;          // live bitmask p x W
+  uint32_t *adj0;         // level 1's snapshot of it for the wide-row kernel, or null
   int *deg;               // snapshot degrees (p)
   int *rowptr;            // snapshot CSR offsets (p + 1)
   int *colidx;            // snapshot neighbour ids, ascending per row
@@ -265,6 +306,14 @@ struct Launch {
   Inst inst0;                       // inst[0] by value: read from the parameter bank when count == 1
   unsigned long long wait_ns;       // bound of the grid barriers' waits (2 s)
   unsigned int bar_extra;           // arrivals added to the barrier target (0; tests raise it)
+  long long p_max;                  // largest p of the launch
+  int wide_cols;                    // columns of an item of the wide level-1 body (a multiple of 32)
+  // level 2's wide rows: the queue's items (front from 0 up, back from wide_cap - 1 down) and
+  // each block's scratch
+  WideItem *wide_items;
+  unsigned int wide_cap;
+  float *wide_scratch;
+  long long wide_floats;
 };
 
 // Instance b's descriptor: the launch's parameter copy for a single instance (no
@@ -395,6 +444,13 @@ long long ctx_retest_queue_bytes(long long sum_p2);
 // entries of re-test scratch for a queue of `cap` items: three per item (a level-1
 // re-test), at most 32 Mi
 long long retest_scratch_entries(long long cap);
+// Whether level 1 runs the wide-row kernel (wide.cuh), from the problems' shapes (p, sum of the
+// degrees after level 0), and the columns of its items.
+struct WideShape {
+  int64_t p, edges2;
+};
+bool wide1_pays(const WideShape *shapes, int count);
+int wide1_cols(const WideShape *shapes, int count);
 // The lowest level whose CI tests run in the set order (citest.cuh; 0: the edge order at
 // every level), process-wide: kSetOrderFrom unless hpc_debug_set_order_from changed it.
 // uses_set_order: whether a level runs in the set order, given the lowest set-order
@@ -448,6 +504,11 @@ struct hpc_ctx {
   void *X_stage = nullptr;        // device copy of host observations
   int64_t X_stage_bytes = 0;
   uint32_t *adj = nullptr;        // sum p * W
+  uint32_t *adj0 = nullptr;       // level 1's snapshot of it (allocated when level 1 first runs on wide rows)
+  hpc::WideItem *wide_items = nullptr;  // level 2's queue of wide rows, allocated likewise
+  long long wide_cap = 0;
+  float *wide_scratch = nullptr;  // ... and its blocks' scratch, wide_floats each
+  long long wide_floats = 0;
   uint8_t *adj_bytes = nullptr;   // p x p expansion for hpc_get_adjacency (largest p)
   int *deg = nullptr;             // sum p
   int *rowptr = nullptr;          // sum (p + 1)
@@ -499,10 +560,19 @@ struct hpc_ctx {
   int p_bucket = 0;
   int citest_grid_l1[3] = {};     // grids of the level-1 kernel variants (kL1*)
   int citest_grid_l1q[2] = {};    // ... and of the queue-only ones (kL1Interleaved, kL1Prefetch | kQueueOnly)
+  int citest_grid_wide[3] = {};   // ... of the wide-row kernels (level 1, 1 queue-only at index 0, level 2)
+  bool wide1 = false, wide2 = false;  // level 1 / level 2 of the runs being queued: the wide-row kernels
+  bool level0_known = false;      // ctr_host holds a level-0 result
+  int wide_cols = 0;              // columns of an item of level 1's
+  int wide_force1 = -1, wide_force2 = -1;  // test hook: 0 / 1 instead of the rules
+  bool wide_denied = false;       // no room for the wide-row kernels' buffers
+  bool tuning = false;            // inside hpc_autotune: a forced policy leaves the wide-row kernels in use
+  int64_t p_max = 0;
   int citest_grid_set[HPC_MAX_LEVEL + 1] = {};  // grids of the set-order kernels (levels 2-16)
   int l1_max_deg = -1;            // level-1 max degree of the last run (keys level 1's kernel choice)
   int l1v_now = 0;                // the level-1 kernel variant of the runs being queued
   int graph_l1v = 0;              // ... and of the captured graph
+  bool graph_wide2 = false;       // ... whose level 2 runs the wide-row kernel
   unsigned int graph_set_mask = 0;  // the set-order levels of the captured graph (bit l)
   int deg_seen[HPC_MAX_LEVEL + 1];  // largest degree at each level's start in the last run (-1: unknown)
   bool set_off = false;           // the set order turned off (a re-test queue overflow)

@@ -88,8 +88,9 @@ __device__ __forceinline__ unsigned long long row_sets(int d, int level) {
 __device__ __forceinline__ bool csr_overflow(const Inst &I) { return (long long)I.rowptr[I.p] > I.colidx_cap; }
 
 // Row i's neighbour list from its adjacency row (whole warp, converged), written
-// ascending at its CSR slot; returns the degree (warp-uniform).
-__device__ __forceinline__ int extract_row(const Inst &I, int64_t i) {
+// ascending at its CSR slot; returns the degree (warp-uniform). snap: the row's words are
+// also kept in adj0.
+__device__ __forceinline__ int extract_row(const Inst &I, int64_t i, bool snap) {
   const int lane = threadIdx.x & 31;
   // the row's first 128 words and its slot offset in one round trip
   const uint32_t *words = I.adj + i * I.W;
@@ -100,6 +101,7 @@ __device__ __forceinline__ int extract_row(const Inst &I, int64_t i) {
   int *out = I.colidx + I.rowptr[i];
   int cnt = 0;
   auto emit = [&](uint32_t word, int w) {
+    if (snap && w < W) I.adj0[i * W + w] = word;
     const int c = __popc(word);
     int incl = c;
 #pragma unroll
@@ -136,7 +138,10 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 // an edge since their last extraction (marked by claim_edge); the other rows keep their
 // lists and degrees. Rows of an instance whose lists overflow their capacity are left
 // alone (the scan phase flags it; the host resizes and reruns).
-__device__ __forceinline__ void rebuild_phase(const Launch &L) {
+// units: what the CI tests are cut by (kUnitTests, kUnitSets, or kUnitNarrow: the tests of the
+// rows below kWideDeg).
+constexpr int kUnitTests = 0, kUnitSets = 1, kUnitNarrow = 2;
+__device__ __forceinline__ void rebuild_phase(const Launch &L, int units, bool snap) {
   const int lane = threadIdx.x & 31;
   const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -191,7 +196,7 @@ __device__ __forceinline__ void rebuild_phase(const Launch &L) {
     while (todo) {
       const int q = __ffs(todo) - 1;
       todo &= todo - 1;
-      const int c = extract_row(*I, i0 + q);
+      const int c = extract_row(*I, i0 + q, snap);
       if (lane == q) cnt = c;
     }
     if (stale) {
@@ -202,7 +207,7 @@ __device__ __forceinline__ void rebuild_phase(const Launch &L) {
     const unsigned long long w = mine ? row_tests(cnt, level, L.row_work_limit, &over) : 0ull;
     a_deg += warp_sum_u64(mine ? (unsigned long long)cnt : 0ull);
     a_work += warp_sum_u64(w);
-    a_sets += warp_sum_u64(w ? row_sets(cnt, level) : 0ull);
+    a_sets += warp_sum_u64(units == kUnitNarrow ? (cnt < kWideDeg ? w : 0ull) : w ? row_sets(cnt, level) : 0ull);
     a_max = max(a_max, __reduce_max_sync(0xffffffffu, mine ? cnt : 0));
     a_rows += (int)__reduce_add_sync(0xffffffffu, w ? 1u : 0u);
     a_over |= (int)__reduce_or_sync(0xffffffffu, (unsigned)over);
@@ -282,7 +287,7 @@ struct InstSums {
 };
 
 // sums over the segments of instance b (one warp); base = units of segments before g
-// (units: tests, or conditioning sets with `set`)
+// (units: the segment's tests, or with `set` its `sets`)
 __device__ __forceinline__ InstSums warp_inst_sums(const Launch &L, int b, long long g, bool set) {
   const int lane = threadIdx.x & 31;
   InstSums r{0, 0, 0, 0, 0, 0, 0};
@@ -311,7 +316,8 @@ __device__ __forceinline__ InstSums warp_inst_sums(const Launch &L, int b, long 
   return r;
 }
 
-__device__ __forceinline__ void scan_phase(const Launch &L, bool set) {
+__device__ __forceinline__ void scan_phase(const Launch &L, int units) {
+  const bool set = units != kUnitTests;
   __shared__ InstSums s_sum;
   __shared__ int s_bad;
   const int level = L.level;
@@ -363,7 +369,14 @@ __device__ __forceinline__ void scan_phase(const Launch &L, bool set) {
     int over = 0;
     const int d = bad ? 0 : d_row;
     unsigned long long w = row_tests(d, level, L.row_work_limit, &over);
-    if (set && w) w = row_sets(d, level);
+    if (units == kUnitSets && w) w = row_sets(d, level);
+    if (units == kUnitNarrow && w && d >= kWideDeg) {  // into the queue of wide rows, the widest first
+      w = 0;
+      const int ns = wide2_slices(d, I.p);
+      const bool first = d >= kWideFirst;
+      const unsigned at = atomicAdd(first ? &L.lc->wide_front : &L.lc->wide_back, (unsigned)ns);
+      for (int q = 0; q < ns; ++q) L.wide_items[first ? at + q : L.wide_cap - 1 - at - q] = WideItem{b, (int32_t)r, q};
+    }
     unsigned long long all;
     const unsigned long long ex = block_exclusive_scan(w, &all);
     if (valid && !bad) I.row_work[r] = s_sum.base + ex;

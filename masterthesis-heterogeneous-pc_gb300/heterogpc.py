@@ -125,6 +125,7 @@ _SIGS = {
     "hpc_debug_set_order_from": (C.c_int, [C.c_int]),
     "hpc_debug_set_retest_queue": (C.c_int, [C.c_void_p, C.c_int64]),
     "hpc_debug_set_order_active": (C.c_int, [C.c_void_p]),
+    "hpc_debug_set_wide": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     "hpc_sem_generate": (C.c_int, [C.POINTER(SemParams), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "hpc_server_opts_default": (C.c_int, [C.POINTER(ServerOpts)]),
     "hpc_server_create": (C.c_int, [C.POINTER(C.c_void_p), C.POINTER(ServerOpts)]),
