@@ -400,6 +400,7 @@ hpc_status collect_level(hpc_ctx *c, int level, hpc_level_stats *out) {
   hpc_level_stats st = level_stats_of(c, level, -1);
   if (level == 1) c->l1_max_deg = st.max_degree;
   if (level >= 1) c->deg_seen[level] = st.max_degree;
+  if (level == 2) c->mean_deg2 = 2.0 * (double)st.edges_before / (double)c->total_rows;
   float t_all = 0.f, t_snap = 0.f, t_test = 0.f, t_re = 0.f;
   if (!c->last_run_graph) {
     HPC_CUDA(cudaEventElapsedTime(&t_snap, c->evl[level][0], c->evl[level][1]));
@@ -521,10 +522,14 @@ hpc_status sync_tune(hpc_ctx *c) {
 
 // Which of levels 1 and 2 run the wide-row kernels (wide.cuh) in the runs being queued, and
 // their buffers: level 1 by the rule on the level-0 result of the context's data (or of its last
-// run), level 2 where rows were much wider than kWideDeg in the last run -- before a first run,
-// where level 1 is wide. (The kernel of level 2 takes the wide rows and leaves the others to the
+// run), level 2 by its degrees in the last run -- before a first run, where level 1 is wide.
+// Level 2 needs kWide2Rows rows of a mean degree of kWide2Deg to keep its blocks busy (measured,
+// ordinary against wide: mean degree 41 of 1000 rows 405 / 455 us, 35 of 700 248 / 508 us; 65 of 1500
+// 1794 / 966 us, 85 of 2000 4.9 / 2.3 ms, 51 of 2000 1.92 / 1.95 ms, 42 of 8000 7.0 / 2.1 ms). (The kernel of level 2 takes the wide rows and leaves the others to the
 // ordinary body, so a wrong guess costs time only.) Without room for the buffers the ordinary
 // kernels run.
+constexpr long long kWide2Rows = 1500;
+constexpr double kWide2Deg = 40.0;
 hpc_status choose_wide(hpc_ctx *c) {
   c->wide1 = c->wide2 = false;
   if (c->opts.precision == HPC_PREC_FP64) return HPC_OK;
@@ -534,7 +539,7 @@ hpc_status choose_wide(hpc_ctx *c) {
     sh[b] = WideShape{c->ih[b].p, c->level0_known ? (int64_t)c->ctr_host[(size_t)b * kLevels].edges2 : 0};
   if (c->level0_known && !forced_policy && !c->wide_denied) {
     c->wide1 = wide1_pays(sh.data(), c->count);
-    c->wide2 = c->deg_seen[2] >= 0 ? c->deg_seen[2] >= 4 * kWideDeg : c->wide1;
+    c->wide2 = c->deg_seen[2] >= 0 ? c->total_rows >= kWide2Rows && c->mean_deg2 >= kWide2Deg : c->wide1;
   }
   if (c->wide_force1 >= 0) c->wide1 = c->wide_force1 > 0;
   if (c->wide_force2 >= 0) c->wide2 = c->wide_force2 > 0;
@@ -922,11 +927,13 @@ bool uses_set_order(int set_from, int level) {
   return set_from > 0 && level >= 2 && level <= kSetTop && level >= set_from;
 }
 
-// Level 1 on wide rows costs a filter step for every variable and pair i < j (sum over the
-// instances of edges2 / 2 * p), the ordinary level-1 body many times that for every potential
-// test (about edges2^2 / p): the wide body where the latter come to kWide1Ratio of the former
-// or more, that is above a mean degree of p / 16, and where there are items for every SM.
-constexpr double kWide1Ratio = 1.0 / 8.0;
+// Level 1 on wide rows costs about 0.8 ns an edge (p up to 3000; 1.1 ns at 9000) and more where
+// the rows hold little of the p variables that it goes over, the ordinary body 2-4 ps an edge and
+// neighbour. Measured, ordinary against wide: mean degree 474 of p = 700 280 / 473 us, 638 of 1000
+// 550 / 503 us, 1029 of 1500 1773 / 634 us, 1645 of 3000 6411 / 1928 us; 444 of 8000 3415 / 4395 us,
+// 237 of 4000 538 / 911 us, a batch of 512 (p up to 800, 42) 3.2 / 3.7 ms. So from a mean degree of
+// kWide1Deg on, where that is an eighth of p or more and there are items for every SM.
+constexpr double kWide1Deg = 600.0, kWide1Density = 1.0 / 8.0;
 static double wide1_items(const WideShape *sh, int count, int cols) {
   double t = 0.0;
   for (int b = 0; b < count; ++b)
@@ -934,13 +941,15 @@ static double wide1_items(const WideShape *sh, int count, int cols) {
   return t;
 }
 bool wide1_pays(const WideShape *sh, int count) {
-  double filter = 0.0, tests = 0.0;
+  double ends = 0.0, deg = 0.0, vars = 0.0;  // edge ends; their rows' mean degrees and p, summed over them
   for (int b = 0; b < count; ++b) {
     const double e2 = (double)sh[b].edges2, p = (double)sh[b].p;
-    filter += 0.5 * e2 * p;
-    tests += e2 * e2 / p;
+    ends += e2;
+    deg += e2 * e2 / p;
+    vars += e2 * p;
   }
-  return tests > kWide1Ratio * filter && wide1_items(sh, count, 256) >= 152.0;
+  return deg >= kWide1Deg * ends && deg >= kWide1Density * vars && ends > 0.0 &&
+         wide1_items(sh, count, 256) >= 152.0;
 }
 // as many columns as leave eight items for every SM (an item's rows are copied once for all of
 // them), 256 (a 32-column word for each warp) at least

@@ -12,23 +12,33 @@
 //                                        all exact in BF16; 49 bits of y)
 //   sum_k y_a y_b = sum_{t+u<=8} 2^-7(t+u) sum_k d_t(a) d_u(b)   (dropped pairs < 2^-56)
 //
-// Each digit product is an integer of at most 2^14, so a sum over 1024 samples is an
-// integer of at most 2^24: exact in the tensor core's FP32 accumulator. The kernel
-// runs, per 128 x 128 tile of the upper triangle, the 28 digit pairs one after another
-// (each a K = n_pad GEMM read by TMA straight from the digit planes), restarts the
-// TMEM accumulator every 1024 samples, and the drain warps add the exact group sums
-// into 64-bit fixed-point integers (LSB 2^-47 of sum y_a y_b) with integer
-// instructions -- the FP64 pipe would be the bottleneck. The epilogue scales by
-// 2^(e_a + e_b) / (n - 1) and writes the FP64 entry (both triangles) and its FP32
-// rounding. Error: the 49-bit digits and the 2^-47 fixed point give |error| below
-// 1e-13 on the correlation for n <= 32768 (the fixed point's range bounds n).
+// Each digit product is an integer of at most 2^14, so sums of a few hundred samples over
+// all the pairs (t, u) of one weight s = t + u are integers of at most 2^24: exact in the
+// tensor core's FP32 accumulator. The kernel keeps one TMEM accumulator per weight and runs
+// a block of 32 samples' digits against each other while they stand in shared memory: 56
+// MMAs for 112 KB of operands, where a pair at a time needs 28 times 16 KB. Seven 128-column
+// accumulators exceed the 512 columns of TMEM, so the samples go by twice: first the weights 2..5
+// (digits 1..4: 10 pairs), then 6..8 (all digits: 18 pairs). Every kGroupStages stages the
+// drain warps add the exact sums into 64-bit fixed-point integers (LSB 2^-47 of sum y_a y_b)
+// with integer instructions -- the FP64 pipe would be the bottleneck -- one weight after the
+// other, while the MMAs of the others go on. Where there are fewer tiles than SMs a cluster of
+// blocks shares a tile's samples and adds up the integers through distributed shared memory:
+// the result does not depend on the split. The epilogue scales by 2^(e_a + e_b) / (n - 1) and
+// writes the FP64 entry (both triangles) and its FP32 rounding. Error: the 49-bit digits and
+// the 2^-47 fixed point give |error| below 1e-13 on the correlation for n <= 32768 (the fixed
+// point's range bounds n).
 //
-// Structure (one CTA of 10 warps per tile, 4-stage shared-memory ring, two 128-column
-// TMEM accumulators): warp 0 lane 0 TMA producer, warp 1 lane 0 MMA issuer
-// (tcgen05.mma.kind::f16, M = N = 128, K = 16), warps 2-9 drain (TMEM lane quadrant
-// warp % 4, 64 columns each). Every mbarrier wait is bounded; on time-out the CTA
-// records kErrTimeout, stops issuing, waits (bounded) for its copies and MMAs, frees
-// its TMEM and returns.
+// Structure (one CTA of 10 warps per tile and part): warp 0 lane 0 TMA producer, warp 1 lane 0
+// MMA issuer (tcgen05.mma.kind::f16, M = N = 128, K = 16), warps 2-9 drain (TMEM lane quadrant
+// warp % 4, 64 columns each). Every mbarrier wait is bounded; on time-out the CTA records
+// kErrTimeout, stops issuing, waits (bounded) for its copies and MMAs, frees its TMEM and
+// returns.
+//
+// Bound: the tensor cores and, beside them, the shared memory they read the operands from
+// (64 of every 80 cycles). Measured (this kernel): p = 2000, n = 5000 918 us with a pair at a
+// time, 497 us now (6.4e11 flops: 1.3 PFLOP/s); p = 1203, n = 3777, on 55 of 152 SMs then, 746 -> 207 us.
+// The digits 616 -> 53 us and 317 -> 27 us.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -38,43 +48,42 @@
 #include "internal.cuh"
 #include "tc_common.cuh"
 
+namespace cg = cooperative_groups;
+
 namespace hpc {
 namespace {
 
-constexpr int EM = 128, EN = 128, EK = 64;   // tile 128 x 128, 64 samples (128 B) per stage
+constexpr int EM = 128, EN = 128, EK = 32;   // tile 128 x 128, 32 samples (64 B of a digit) per stage
 constexpr int kDigits = 7;
-constexpr int kPairs = 28;                   // (t, u), t + u <= 8 (1-based)
-constexpr int kGroupKb = 16;                 // k-blocks per exact group: 1024 samples
-constexpr int kSampleAlign = EK * kGroupKb;  // n is padded to whole groups
-constexpr int kStagesE = 4;
-constexpr int kStageBytesE = (EM + EN) * EK * 2;  // 32 KB
-constexpr int kTmemColsE = 256;              // two 128-column accumulators
+constexpr int kTileBytes = EM * EK * 2;      // one digit's 128 rows of a stage: 8 KB
+// The two passes: weights s = 2..5 and 6..8 (accumulators 0..3 and 0..2), the digits they
+// need, and their stages -- both cut the same 224 KB.
+constexpr int kDigitsA = 4, kSlotsA = 4, kStagesA = 3, kBytesA = 2 * kDigitsA * kTileBytes;
+constexpr int kDigitsB = 7, kSlotsB = 3, kStagesB = 2, kBytesB = 2 * kDigitsB * kTileBytes;
+constexpr int kOperandBytes = kStagesB * kBytesB;
+static_assert(kStagesA * kBytesA <= kOperandBytes, "both passes share the operand buffer");
+// Stages between two drains: the largest weight's sum grows by (2 * 2^13 + 5 * 2^12) a sample at
+// most (d_1 against d_7 twice, |d_1| <= 128, and five pairs of |d| <= 64), so 448 samples
+// stay below 2^24
+constexpr int kGroupStages = 14;
+static_assert((2 * 8192 + 5 * 4096) * kGroupStages * EK <= (1 << 24), "exact in FP32");
+constexpr int kTmemColsE = 512;              // four 128-column accumulators
 constexpr int kAccWarpsE = 8;
 constexpr int kThreadsE = 64 + 32 * kAccWarpsE;
 constexpr int kFixL = 47;                    // fixed-point LSB 2^-47
-
-// digit pair q -> 0-based digits (t, u) with t + u = s - 2, pairs ordered by s = 2..8
-__device__ __forceinline__ void emu_pair(int q, int *t, int *u, int *s) {
-  int ss = 2;
-  while (q >= ss - 1) {
-    q -= ss - 1;
-    ++ss;
-  }
-  *t = q;
-  *u = ss - 2 - q;
-  *s = ss;
-}
+constexpr int kMaxSplitE = 8;                // portable cluster size
 
 struct alignas(1024) EmuSmem {
-  uint8_t stage[kStagesE][kStageBytesE];
-  uint64_t full[kStagesE];
-  uint64_t empty[kStagesE];
-  uint64_t acc_full[2];
-  uint64_t acc_empty[2];
+  uint8_t operands[kOperandBytes];  // the stages; at the end a block's 128 x 128 integer sums
+  uint64_t full_a[kStagesA], empty_a[kStagesA];
+  uint64_t full_b[kStagesB], empty_b[kStagesB];
+  uint64_t acc_full[kSlotsA], acc_empty[kSlotsA];
   uint64_t drain;
   uint32_t tmem_base;
   int abort;
 };
+static_assert(sizeof(EmuSmem) + 1024 <= 227 * 1024, "shared memory of a block");
+static_assert(sizeof(long long) * EM * EN <= kOperandBytes, "the sums fit the operand buffer");
 
 __device__ __forceinline__ bool aborted(EmuSmem &sm) { return *(volatile int *)&sm.abort != 0; }
 __device__ __forceinline__ void fail(EmuSmem &sm, int *err) {
@@ -82,72 +91,104 @@ __device__ __forceinline__ void fail(EmuSmem &sm, int *err) {
   atomicExch(&sm.abort, 1);
 }
 
-// One block per variable (rows beyond p are written as zero digits): the exponent of
-// max |z| and the seven digits of z * 2^-e for every sample (zero beyond n).
+// One block per variable (rows beyond p are written as zero digits): the exponent of max |z|
+// and the seven digits of z * 2^-e for every sample (zero beyond n, and for a sample that is
+// not finite). All in integers on the bits of z -- rounded to 49 bits, then cut 7 bits at a
+// time -- since the FP64 pipe (2 results a clock and SM) took 616 us for p = 2000, n = 5000 where
+// the 220 MB of traffic take 32. Four samples a thread, so that a digit's four go out as 8 bytes.
 __global__ void __launch_bounds__(256) emu_digits_kernel(const double *__restrict__ Z, int64_t p, int64_t n,
                                                          int64_t n_pad, __nv_bfloat16 *__restrict__ D,
                                                          int *__restrict__ E) {
   const int64_t v = blockIdx.x;
   __nv_bfloat16 *dv = D + v * (int64_t)kDigits * n_pad;
-  __shared__ double red[8];
-  __shared__ int s_e;
+  const long long *zv = reinterpret_cast<const long long *>(Z + v * n);
+  __shared__ int red[8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  double m = 0.0;
+  int ex = 0;  // largest biased exponent of a finite sample (0: all zero or denormal)
   if (v < p)
-    for (int64_t k = threadIdx.x; k < n; k += blockDim.x) m = fmax(m, fabs(Z[v * n + k]));
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) red[wid] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double mm = 0.0;
-    for (int w = 0; w < 8; ++w) mm = fmax(mm, red[w]);
-    int e = 0;
-    if (mm > 0.0) frexp(mm, &e);  // mm = f 2^e, f in [0.5, 1): 2^e > mm
-    s_e = e;
-    E[v] = e;
-  }
-  __syncthreads();
-  const int e = s_e;
-  for (int64_t k = threadIdx.x; k < n_pad; k += blockDim.x) {
-    double r = (v < p && k < n) ? ldexp(Z[v * n + k], 7 - e) : 0.0;  // 128 y, exact
-#pragma unroll
-    for (int t = 0; t < kDigits; ++t) {
-      const double d = rint(r);  // |d| <= 128, an integer: exact in BF16
-      dv[t * n_pad + k] = __double2bfloat16(d);
-      r = (r - d) * 128.0;       // exact: the remainder and a power of two
+    for (int64_t k = threadIdx.x; k < n; k += blockDim.x) {
+      const int x = (int)(__ldg(zv + k) >> 52) & 0x7ff;
+      if (x < 0x7ff) ex = max(ex, x);
     }
+  ex = __reduce_max_sync(0xffffffffu, ex);
+  if (lane == 0) red[wid] = ex;
+  __syncthreads();
+  int e = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) e = max(e, red[w]);
+  e = e ? e - 1022 : 0;  // max |z| = f 2^e, f in [0.5, 1)
+  if (threadIdx.x == 0) E[v] = e;
+  for (int64_t k = 4 * (int64_t)threadIdx.x; k < n_pad; k += 4 * blockDim.x) {
+    uint32_t dig[kDigits][4];  // FP32 bits of the digits: small integers, exact in their upper half
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long bits = v < p && k + u < n ? __ldg(zv + k + u) : 0ll;
+      const int x = (int)(bits >> 52) & 0x7ff;
+      // N = rint(|z| 2^(49 - e)): the 53-bit mantissa shifted right by sh >= 4, to nearest even
+      const int sh = 1026 + e - x;
+      const unsigned long long m = ((unsigned long long)bits & 0xfffffffffffffull) | (1ull << 52);
+      long long N = 0;
+      if (x != 0 && x != 0x7ff && sh < 60)
+        N = (long long)((m + ((1ull << (sh - 1)) - 1ull) + ((m >> sh) & 1ull)) >> sh);
+      if (bits < 0) N = -N;
+      // digits 7..5 in 64 bits, the other 28 bits in 32
+#pragma unroll
+      for (int t = kDigits - 1; t >= 4; --t) {
+        const int d = ((int)(N + 64) & 127) - 64;
+        N = (N - d) >> 7;
+        dig[t][u] = __float_as_uint((float)d);
+      }
+      int M = (int)N;
+#pragma unroll
+      for (int t = 3; t >= 1; --t) {
+        const int d = ((M + 64) & 127) - 64;
+        M = (M - d) >> 7;
+        dig[t][u] = __float_as_uint((float)d);
+      }
+      dig[0][u] = __float_as_uint((float)M);
+    }
+#pragma unroll
+    for (int t = 0; t < kDigits; ++t)
+      *reinterpret_cast<uint2 *>(dv + t * n_pad + k) =
+          make_uint2(__byte_perm(dig[t][0], dig[t][1], 0x7632), __byte_perm(dig[t][2], dig[t][3], 0x7632));
   }
 }
 
 __global__ void __launch_bounds__(kThreadsE, 1)
     gram_emu_kernel(const __grid_constant__ CUtensorMap map, int64_t p, int64_t n_pad, double denom,
-                    const int *__restrict__ E, double *__restrict__ C64, float *__restrict__ C32, int *err) {
+                    const int *__restrict__ E, double *__restrict__ C64, float *__restrict__ C32, int *err, int split) {
   extern __shared__ uint8_t smem_raw[];
   EmuSmem &sm = *reinterpret_cast<EmuSmem *>((((uintptr_t)smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // tile (bi, bj), bi <= bj, row-major over the upper triangle of 128-blocks
+  // tile (bi, bj), bi <= bj, row-major over the upper triangle of 128-blocks, and the block's part
+  // of the samples
   const int nb = (int)((p + EM - 1) / EM);
-  long long t = blockIdx.x;
+  const int part = (int)(blockIdx.x % (unsigned)split);
+  long long t = blockIdx.x / (unsigned)split;
   int bi = 0;
   while (t >= nb - bi) {
     t -= nb - bi;
     ++bi;
   }
   const int bj = bi + (int)t;
-  const int kbp = (int)(n_pad / EK);         // k-blocks per digit pair
-  const int kblocks = kPairs * kbp;
-  const int groups = kblocks / kGroupKb;
-  const int gpp = kbp / kGroupKb;            // groups per pair
+  const int stages = (int)(n_pad / EK);
+  const int kb0 = (int)((long long)stages * part / split), kb1 = (int)((long long)stages * (part + 1) / split);
+  const int nk = kb1 - kb0;
+  const int groups = (nk + kGroupStages - 1) / kGroupStages;
   const uint32_t idesc = idesc_bf16(EM, EN);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStagesE; ++s) {
-      mbar_init(&sm.full[s], 1);
-      mbar_init(&sm.empty[s], 1);
+    for (int s = 0; s < kStagesA; ++s) {
+      mbar_init(&sm.full_a[s], 1);
+      mbar_init(&sm.empty_a[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&sm.acc_full[b], 1);
-      mbar_init(&sm.acc_empty[b], kAccWarpsE);
+    for (int s = 0; s < kStagesB; ++s) {
+      mbar_init(&sm.full_b[s], 1);
+      mbar_init(&sm.empty_b[s], 1);
+    }
+    for (int c = 0; c < kSlotsA; ++c) {
+      mbar_init(&sm.acc_full[c], 1);
+      mbar_init(&sm.acc_empty[c], kAccWarpsE);
     }
     mbar_init(&sm.drain, 1);
     sm.abort = 0;
@@ -162,109 +203,174 @@ __global__ void __launch_bounds__(kThreadsE, 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = sm.tmem_base;
 
-  int issued = 0;
+  int issued_a = 0, issued_b = 0;
+  constexpr int kCols = EN / 2;
+  long long acc[kCols];  // drain warps: the thread's row, 64 columns
+  bool ok = true;
   if (warp == 0 && lane == 0) {
-    // TMA producer: pair q's k-block kb of digit t (rows of block bi) and u (block bj)
-    for (int kg = 0; kg < kblocks; ++kg) {
-      const int s = kg % kStagesE;
-      if (kg >= kStagesE && !mbar_wait(&sm.empty[s], ((kg / kStagesE) + 1) & 1)) {
+    // TMA producer: each stage's digits of the rows (block bi) and of the columns (block bj)
+    auto load = [&](uint8_t *to, int digits, int kb, uint64_t *bar) {
+      for (int d = 0; d < digits; ++d) {
+        tma_load_2d(to + d * kTileBytes, &map, (int)(d * n_pad) + kb * EK, bi * EM, bar);
+        tma_load_2d(to + (digits + d) * kTileBytes, &map, (int)(d * n_pad) + kb * EK, bj * EN, bar);
+      }
+    };
+    for (int k = 0; k < nk; ++k) {
+      const int s = k % kStagesA;
+      if (k >= kStagesA && !mbar_wait(&sm.empty_a[s], ((k / kStagesA) + 1) & 1)) {
         fail(sm, err);
         break;
       }
       if (aborted(sm)) break;
-      int dt, du, ss;
-      emu_pair(kg / kbp, &dt, &du, &ss);
-      const int kb = kg % kbp;
-      mbar_arrive_expect_tx(&sm.full[s], kStageBytesE);
-      tma_load_2d(sm.stage[s], &map, (int)(dt * n_pad) + kb * EK, bi * EM, &sm.full[s]);
-      tma_load_2d(sm.stage[s] + EM * EK * 2, &map, (int)(du * n_pad) + kb * EK, bj * EN, &sm.full[s]);
-      ++issued;
+      mbar_arrive_expect_tx(&sm.full_a[s], kBytesA);
+      load(sm.operands + s * kBytesA, kDigitsA, kb0 + k, &sm.full_a[s]);
+      ++issued_a;
     }
-  } else if (warp == 1 && lane == 0) {
-    // MMA issuer: group g (1024 samples of one digit pair) into TMEM buffer g % 2
-    for (int g = 0; g < groups && !aborted(sm); ++g) {
-      const int b = g & 1;
-      if (g >= 2 && !mbar_wait(&sm.acc_empty[b], ((g >> 1) + 1) & 1)) {
+    // the second pass overwrites the first one's stages: all of them have been read
+    for (int s = 0; s < kStagesA && !aborted(sm); ++s) {
+      const int fills = issued_a / kStagesA + (s < issued_a % kStagesA ? 1 : 0);
+      if (fills > 0 && !mbar_wait(&sm.empty_a[s], (fills - 1) & 1)) fail(sm, err);
+    }
+    for (int k = 0; k < nk && !aborted(sm); ++k) {
+      const int s = k % kStagesB;
+      if (k >= kStagesB && !mbar_wait(&sm.empty_b[s], ((k / kStagesB) + 1) & 1)) {
         fail(sm, err);
         break;
       }
-      const uint32_t dcol = tmem + (uint32_t)(b * EN);
-      for (int kg = g * kGroupKb; kg < (g + 1) * kGroupKb; ++kg) {
-        const int s = kg % kStagesE;
-        if (!mbar_wait(&sm.full[s], (kg / kStagesE) & 1)) {
+      if (aborted(sm)) break;
+      mbar_arrive_expect_tx(&sm.full_b[s], kBytesB);
+      load(sm.operands + s * kBytesB, kDigitsB, kb0 + k, &sm.full_b[s]);
+      ++issued_b;
+    }
+  } else if (warp == 1 && lane == 0) {
+    // MMA issuer. Pass P: accumulator c takes the digit pairs of weight first + c; a stage's MMAs of
+    // one accumulator after the other, so that a drained one is refilled while the next is drained.
+    // fill: how often the accumulators were filled before (their barriers' phases)
+    auto run = [&](int first, int slots, int digits, int nstages, int bytes, uint64_t *full, uint64_t *empty,
+                   int fill) {
+      for (int k = 0; k < nk && !aborted(sm); ++k) {
+        const int s = k % nstages, g = k / kGroupStages;
+        const bool begin = k % kGroupStages == 0, end = k == nk - 1 || (k + 1) % kGroupStages == 0;
+        if (!mbar_wait(&full[s], (k / nstages) & 1)) {
           fail(sm, err);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = smem_u32(sm.stage[s]), b0 = a0 + EM * EK * 2;
+        const uint32_t a0 = smem_u32(sm.operands + s * bytes), b0 = a0 + digits * kTileBytes;
+        for (int c = 0; c < slots; ++c) {
+          if (begin && fill + g > 0) {
+            if (!mbar_wait(&sm.acc_empty[c], (fill + g - 1) & 1)) {
+              fail(sm, err);
+              break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          }
+          const int sum = first - 2 + c;  // 0-based digits t + u
+          for (int t0 = 0; t0 <= sum; ++t0) {
+            const uint32_t a = a0 + t0 * kTileBytes, bb = b0 + (sum - t0) * kTileBytes;
 #pragma unroll
-        for (int k = 0; k < EK / 16; ++k)
-          mma_bf16(dcol, smem_desc_sw128(a0 + k * 32), smem_desc_sw128(b0 + k * 32), idesc,
-                   (kg > g * kGroupKb || k > 0) ? 1u : 0u);
-        mma_commit(&sm.empty[s]);
+            for (int kk = 0; kk < EK / 16; ++kk)
+              mma_bf16(tmem + (uint32_t)(c * EN), smem_desc_sw64(a + kk * 32), smem_desc_sw64(bb + kk * 32), idesc,
+                       (begin && t0 == 0 && kk == 0) ? 0u : 1u);
+          }
+          if (end) mma_commit(&sm.acc_full[c]);
+        }
+        mma_commit(&empty[s]);
       }
-      mma_commit(&sm.acc_full[b]);
-    }
+    };
+    run(2, kSlotsA, kDigitsA, kStagesA, kBytesA, sm.full_a, sm.empty_a, 0);
+    run(2 + kSlotsA, kSlotsB, kDigitsB, kStagesB, kBytesB, sm.full_b, sm.empty_b, groups);
     mma_commit(&sm.drain);
     if (!mbar_wait(&sm.drain, 0)) fail(sm, err);
   } else if (warp >= 2) {
     // drain: rows 32 (warp % 4) .. + 31 (TMEM lanes), columns 64 ((warp - 2) / 4) .. + 63
     const int quad = warp & 3;
     const int half = (warp - 2) >> 2;
-    constexpr int kCols = EN / 2;
-    long long acc[kCols];
 #pragma unroll
     for (int q = 0; q < kCols; ++q) acc[q] = 0;
-    bool ok = true;
-    for (int g = 0; g < groups; ++g) {
-      const int b = g & 1;
-      if (!mbar_wait(&sm.acc_full[b], (g >> 1) & 1)) {
-        fail(sm, err);
-        ok = false;
-        break;
-      }
-      __syncwarp();
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      int dt, du, ss;
-      emu_pair(g / gpp, &dt, &du, &ss);
-      const int sh = kFixL - 7 * ss;  // the group sum's weight 2^-7s in units of 2^-47
-#pragma unroll
-      for (int c0 = 0; c0 < kCols; c0 += 32) {
-        float v[32];
-        tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * EN + half * kCols + c0), v);
-#pragma unroll
-        for (int q = 0; q < 32; ++q) {
-          const long long gi = (long long)__float2int_rn(v[q]);  // an integer below 2^24: exact
-          acc[c0 + q] += sh >= 0 ? gi * (1ll << sh) : (gi >> (-sh));
-        }
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.acc_empty[b]);
-    }
-    if (ok && !aborted(sm)) {
-      const int64_t row = (int64_t)bi * EM + quad * 32 + lane;
-      const int64_t col0 = (int64_t)bj * EN + half * kCols;
-      const int er = row < p ? E[row] : 0;
-#pragma unroll 4
-      for (int cc = 0; cc < kCols; ++cc) {
-        const int64_t col = col0 + cc;
-        if (row < p && col < p && col >= row) {
-          const double v = ldexp((double)acc[cc], er + E[col] - kFixL) / denom;
-          C64[col * p + row] = v;  // the warp's lanes: consecutive rows, one column
-          C64[row * p + col] = v;
-          if (C32) {
-            C32[col * p + row] = (float)v;
-            C32[row * p + col] = (float)v;
+    for (int pass = 0; pass < 2 && ok; ++pass) {
+      const int slots = pass ? kSlotsB : kSlotsA, first = pass ? 2 + kSlotsA : 2;
+      for (int g = 0; g < groups && ok; ++g)
+        for (int c = 0; c < slots; ++c) {
+          if (!mbar_wait(&sm.acc_full[c], (pass * groups + g) & 1)) {
+            fail(sm, err);
+            ok = false;
+            break;
           }
+          __syncwarp();
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const int sh = kFixL - 7 * (first + c);  // the sum's weight 2^-7s in units of 2^-47
+#pragma unroll
+          for (int c0 = 0; c0 < kCols; c0 += 16) {
+            float v[16];
+            tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * EN + half * kCols + c0), v);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+              const long long gi = (long long)__float2int_rn(v[q]);  // an integer of at most 2^24: exact
+              acc[c0 + q] += sh >= 0 ? (long long)((unsigned long long)gi << sh) : (gi >> (-sh));
+            }
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.acc_empty[c]);
         }
-      }
     }
   }
+  __syncwarp();
+  // one entry: scaled, both triangles. 1 / denom times a power of two: one multiplication (a
+  // division's FP64 instructions would take 40 us at p = 2000)
+  const double inv = 1.0 / denom;
+  auto write = [&](int64_t row, int64_t col, long long sum, int er) {
+    if (row < p && col < p && col >= row) {
+      const double scale = __hiloint2double(__double2hiint(inv) + ((er + E[col] - kFixL) << 20), __double2loint(inv));
+      const double v = (double)sum * scale;
+      C64[col * p + row] = v;  // the warp's lanes: consecutive rows, one column
+      C64[row * p + col] = v;
+      if (C32) {
+        C32[col * p + row] = (float)v;
+        C32[row * p + col] = (float)v;
+      }
+    }
+  };
+  const int64_t row = (int64_t)bi * EM + (warp & 3) * 32 + lane;
+  const int er = warp >= 2 && row < p ? E[row] : 0;
+  if (split == 1) {
+    if (warp >= 2 && ok && !aborted(sm)) {
+      const int64_t col0 = (int64_t)bj * EN + ((warp - 2) >> 2) * kCols;
+#pragma unroll
+      for (int cc = 0; cc < kCols; ++cc) write(row, col0 + cc, acc[cc], er);
+    }
+  } else {
+    // the parts' sums: each block keeps its own in its operand buffer (every copy and MMA has
+    // completed), then adds up and writes its share of the columns
+    cg::cluster_group cluster = cg::this_cluster();
+    long long *sums = reinterpret_cast<long long *>(sm.operands);  // [column][row]
+    __syncthreads();
+    if (warp >= 2) {
+      const int c0 = ((warp - 2) >> 2) * kCols, r = (warp & 3) * 32 + lane;
+#pragma unroll
+      for (int cc = 0; cc < kCols; ++cc) sums[(c0 + cc) * EM + r] = acc[cc];
+    }
+    cluster.sync();
+    if (warp >= 2 && !aborted(sm)) {  // a part that failed has raised err: the host does not use C
+      const int r = (warp & 3) * 32 + lane;
+      const int lo = EN * part / split, hi = EN * (part + 1) / split;
+      for (int cc = lo + ((warp - 2) >> 2); cc < hi; cc += 2) {
+        long long sum = 0;
+        for (int q = 0; q < split; ++q) sum += cluster.map_shared_rank(sums, q)[cc * EM + r];
+        write(row, (int64_t)bj * EN + cc, sum, er);
+      }
+    }
+    cluster.sync();  // no block leaves while its sums are read
+  }
   if (warp == 0 && lane == 0 && sm.abort) {
-    for (int s = 0; s < kStagesE; ++s) {
-      const int fills = issued / kStagesE + (s < issued % kStagesE ? 1 : 0);
-      if (fills > 0) mbar_wait(&sm.full[s], (fills - 1) & 1);
+    for (int s = 0; s < kStagesA; ++s) {
+      const int fills = issued_a / kStagesA + (s < issued_a % kStagesA ? 1 : 0);
+      if (fills > 0) mbar_wait(&sm.full_a[s], (fills - 1) & 1);
+    }
+    for (int s = 0; s < kStagesB; ++s) {
+      const int fills = issued_b / kStagesB + (s < issued_b % kStagesB ? 1 : 0);
+      if (fills > 0) mbar_wait(&sm.full_b[s], (fills - 1) & 1);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -274,7 +380,15 @@ __global__ void __launch_bounds__(kThreadsE, 1)
   }
 }
 
-int64_t emu_n_pad(int64_t n) { return (n + kSampleAlign - 1) / kSampleAlign * kSampleAlign; }
+int64_t emu_n_pad(int64_t n) { return (n + EK - 1) / EK * EK; }
+
+// Blocks a tile's samples are split over: the largest power of two (up to a portable cluster)
+// with which every block still runs at once, one an SM, and keeps a group of stages or more.
+int emu_split(long long tiles, int64_t n_pad) {
+  int split = 1;
+  while (split < kMaxSplitE && tiles * split * 2 <= 152 && n_pad / (split * 2) >= kGroupStages * EK) split *= 2;
+  return split;
+}
 
 }  // namespace
 
@@ -290,13 +404,25 @@ hpc_status launch_gram_emu(const double *Z, int64_t p, int64_t n, double denom, 
   emu_digits_kernel<<<(unsigned)p_pad, 256, 0, s>>>(Z, p, n, n_pad, D, E);
   HPC_LAUNCH_CHECK("emu_digits_kernel");
   CUtensorMap map;
-  hpc_status st = tc_make_map(&map, D, p_pad, kDigits * n_pad, EM);
+  hpc_status st = tc_make_map(&map, D, p_pad, kDigits * n_pad, EM, EK);
   if (st != HPC_OK) return st;
   const int smem = (int)sizeof(EmuSmem) + 1024;
   HPC_CUDA(cudaFuncSetAttribute(gram_emu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const long long nb = p_pad / EM, tiles = nb * (nb + 1) / 2;
-  gram_emu_kernel<<<(unsigned)tiles, kThreadsE, smem, s>>>(map, p, n_pad, denom, E, C64, C32, err);
-  HPC_LAUNCH_CHECK("gram_emu_kernel");
+  const int split = emu_split(tiles, n_pad);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * split));
+  cfg.blockDim = dim3(kThreadsE);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  HPC_CUDA(cudaLaunchKernelEx(&cfg, gram_emu_kernel, map, p, n_pad, denom, (const int *)E, C64, C32, err, split));
   return HPC_OK;
 }
 

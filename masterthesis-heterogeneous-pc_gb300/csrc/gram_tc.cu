@@ -291,7 +291,7 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-hpc_status make_map(CUtensorMap *m, const __nv_bfloat16 *base, int64_t rows, int64_t K, int box_rows) {
+hpc_status make_map(CUtensorMap *m, const __nv_bfloat16 *base, int64_t rows, int64_t K, int box_rows, int box_k) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) {
     set_error("cuTensorMapEncodeTiled is not available from the driver");
@@ -299,10 +299,11 @@ hpc_status make_map(CUtensorMap *m, const __nv_bfloat16 *base, int64_t rows, int
   }
   cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)(K * 2)};
-  cuuint32_t box[2] = {(cuuint32_t)TK, (cuuint32_t)box_rows};
+  cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)base, dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, box_k == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled failed (%d)", (int)r);
@@ -326,17 +327,17 @@ long long gram_tc_tiles(int64_t p) {
 
 // Tensor maps of one instance's operand planes (tc_p_pad(p) rows of tc_k(n) bf16), for
 // the A (128-row) and B (256-row) tiles; P and Q may be the same buffer.
-// a 2-D BF16 tensor map (rows x K, K contiguous, 64-column x box_rows boxes, 128-byte
-// swizzle) for the other tensor-core kernels
-hpc_status tc_make_map(CUtensorMap *m, const __nv_bfloat16 *base, int64_t rows, int64_t K, int box_rows) {
-  return make_map(m, base, rows, K, box_rows);
+// a 2-D BF16 tensor map (rows x K, K contiguous, boxes of box_rows rows and box_k = 32 or 64
+// columns with a swizzle of as many bytes twice) for the other tensor-core kernels
+hpc_status tc_make_map(CUtensorMap *m, const __nv_bfloat16 *base, int64_t rows, int64_t K, int box_rows, int box_k) {
+  return make_map(m, base, rows, K, box_rows, box_k);
 }
 
 hpc_status tc_make_maps(CUtensorMap *mp, CUtensorMap *mq, const __nv_bfloat16 *P, const __nv_bfloat16 *Q,
                         int64_t p, int64_t n) {
   hpc_status st;
-  if ((st = make_map(mp, P, tc_p_pad(p), tc_k(n), TM)) != HPC_OK) return st;
-  return make_map(mq, Q, tc_p_pad(p), tc_k(n), TN);
+  if ((st = make_map(mp, P, tc_p_pad(p), tc_k(n), TM, TK)) != HPC_OK) return st;
+  return make_map(mq, Q, tc_p_pad(p), tc_k(n), TN, TK);
 }
 
 // C (p x p FP32 per instance, row-major) = P Q^T over upper-triangle tiles, mirrored;

@@ -392,7 +392,7 @@ struct TcArgs {                     // grouped tensor-core Gram
   int *err;
 };
 hpc_status launch_gram_tc(float *C, const TcArgs &a, long long total_tiles, cudaStream_t s);
-hpc_status tc_make_map(CUtensorMap *m, const __nv_bfloat16 *base, int64_t rows, int64_t K, int box_rows);
+hpc_status tc_make_map(CUtensorMap *m, const __nv_bfloat16 *base, int64_t rows, int64_t K, int box_rows, int box_k);
 // FP64-accurate Gram on the tensor cores (gram_emu.cu): C64 (and C32 when not null) =
 // Z^T Z / denom for one instance's standardised data Z (n x p, each variable
 // contiguous). D (digits) and E (exponents) are its work buffers of emu_digit_elems /
@@ -565,6 +565,7 @@ struct hpc_ctx {
   bool level0_known = false;      // ctr_host holds a level-0 result
   int wide_cols = 0;              // columns of an item of level 1's
   int wide_force1 = -1, wide_force2 = -1;  // test hook: 0 / 1 instead of the rules
+  double mean_deg2 = 0.0;         // mean degree at level 2's start in the last run
   bool wide_denied = false;       // no room for the wide-row kernels' buffers
   bool tuning = false;            // inside hpc_autotune: a forced policy leaves the wide-row kernels in use
   int64_t p_max = 0;
