@@ -138,6 +138,79 @@ __device__ __noinline__ double partial_r_of_matrix(double *M, int l, bool *nan_p
   return -p01 / sqrt(p00 * p11);
 }
 
+// partial_r_of_matrix from an instance's FP64 matrix with everything in registers, for levels
+// 2..LA (unrolled): the same operations in the same order. *ok is false where that takes the
+// pseudoinverse (the caller then goes through partial_r_of_matrix).
+template <int LA>
+__device__ __forceinline__ double partial_r_registers(const Inst &I, int64_t i, int64_t j, const int *ids, int l,
+                                                      bool *nan_p, bool *ok) {
+  const double *C = I.cor64;
+  const int64_t p = I.p;
+  const double rij = C[i * p + j];
+  double gx[LA], gy[LA], gs[LA * (LA - 1) / 2];
+  bool nan_in = isnan(rij);
+#pragma unroll
+  for (int r = 0; r < LA; ++r)
+    if (r < l) {
+      const int64_t idr = ids[r];
+      gx[r] = C[i * p + idr];
+      gy[r] = C[j * p + idr];
+      nan_in |= isnan(gx[r]) || isnan(gy[r]);
+#pragma unroll
+      for (int c = 0; c < r; ++c) {
+        gs[r * (r - 1) / 2 + c] = C[(int64_t)ids[c] * p + idr];
+        nan_in |= isnan(gs[r * (r - 1) / 2 + c]);
+      }
+    }
+  *nan_p = nan_in;
+  *ok = true;
+  if (nan_in) return 0.0;
+  double Lm[LA * (LA + 1) / 2], wx[LA], wy[LA];
+  double dmin = 1.0;
+#pragma unroll
+  for (int r = 0; r < LA; ++r)
+    if (r < l && dmin > 1e-10) {
+#pragma unroll
+      for (int c = 0; c < r; ++c) {
+        double v = gs[r * (r - 1) / 2 + c];
+#pragma unroll
+        for (int q = 0; q < c; ++q) v -= Lm[r * (r + 1) / 2 + q] * Lm[c * (c + 1) / 2 + q];
+        Lm[r * (r + 1) / 2 + c] = v / Lm[c * (c + 1) / 2 + c];
+      }
+      double d = 1.0;
+#pragma unroll
+      for (int q = 0; q < r; ++q) d -= Lm[r * (r + 1) / 2 + q] * Lm[r * (r + 1) / 2 + q];
+      dmin = fmin(dmin, d);
+      if (d > 1e-10) {
+        const double lrr = sqrt(d);
+        Lm[r * (r + 1) / 2 + r] = lrr;
+        double vx = gx[r], vy = gy[r];
+#pragma unroll
+        for (int q = 0; q < r; ++q) {
+          vx -= Lm[r * (r + 1) / 2 + q] * wx[q];
+          vy -= Lm[r * (r + 1) / 2 + q] * wy[q];
+        }
+        wx[r] = vx / lrr;
+        wy[r] = vy / lrr;
+      } else {
+        dmin = 0.0;
+      }
+    }
+  if (dmin > 1e-10) {
+    double ax = 1.0, ay = 1.0, b = rij;
+#pragma unroll
+    for (int q = 0; q < LA; ++q)
+      if (q < l) {
+        ax -= wx[q] * wx[q];
+        ay -= wy[q] * wy[q];
+        b -= wx[q] * wy[q];
+      }
+    if (ax > 1e-10 && ay > 1e-10) return b / sqrt(ax * ay);
+  }
+  *ok = false;
+  return 0.0;
+}
+
 // FP64 p-value of a k x k submatrix M with the reference's semantics.
 template <int LA>
 __device__ __forceinline__ double pvalue_of_matrix(double *M, int l, int n_obs) {
