@@ -2,6 +2,7 @@
 // instantiations of levels 1-8 and the launchers (the level kernels' device code is in
 // citest.cuh, wide.cuh and level_kernel.cuh).
 #include <algorithm>
+#include <atomic>
 
 #include "level_kernel.cuh"
 
@@ -471,15 +472,31 @@ int level_smem(int level, int variant) {
 
 }  // namespace
 
+// Blocks of a level kernel that are resident at once. Asked of the driver once per device and
+// kernel (a context asks for up to 60, which took a third of its creation).
 int citest_grid(int precision, int level, int device, int l1_variant) {
-  void *k = precision == HPC_PREC_FP64 ? kernel_for<false>(level, l1_variant) : kernel_for<true>(level, l1_variant);
+  constexpr int kDevices = 64, kVariants = 16;
+  static std::atomic<int> known[kDevices][2][HPC_MAX_LEVEL + 1][kVariants];
+  const bool mixed = precision != HPC_PREC_FP64;
+  std::atomic<int> *slot = device >= 0 && device < kDevices && l1_variant >= 0 && l1_variant < kVariants
+                               ? &known[device][mixed ? 1 : 0][level][l1_variant] : nullptr;
+  if (slot)
+    if (const int g = slot->load(std::memory_order_acquire)) return g;
+  void *k = mixed ? kernel_for<true>(level, l1_variant) : kernel_for<false>(level, l1_variant);
   const int smem = level_smem(level, l1_variant);
   // beyond the default 48 KB of shared memory
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) cudaGetLastError();
   int per_sm = 0, sms = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem) != cudaSuccess || per_sm < 1)
+  bool ok = true;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem) != cudaSuccess || per_sm < 1) {
     per_sm = 1;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 1) sms = 1;
+    ok = false;
+  }
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 1) {
+    sms = 1;
+    ok = false;
+  }
+  if (slot && ok) slot->store(per_sm * sms, std::memory_order_release);
   return per_sm * sms;
 }
 

@@ -153,6 +153,25 @@ double denom_of(const hpc_ctx *c, int64_t n) {
   return c->opts.ref_compat_sd ? (double)((float)n - 1.f) : (double)(n - 1);
 }
 
+// A small value to device memory in stream order, as a kernel's parameter: unlike a copy it
+// leaves no host memory to keep until it is done, so nothing waits for it.
+template <typename T>
+__global__ void put_kernel(T *dst, const __grid_constant__ T v) {
+  static_assert(sizeof(T) % 4 == 0 && sizeof(T) <= 1024, "a few hundred bytes");
+  for (unsigned w = threadIdx.x; w < sizeof(T) / 4; w += blockDim.x)
+    reinterpret_cast<uint32_t *>(dst)[w] = reinterpret_cast<const uint32_t *>(&v)[w];
+}
+template <int N>
+struct Words {
+  long long w[N];
+};
+template <typename T>
+hpc_status put(T *dst, const T &v, cudaStream_t s) {
+  put_kernel<T><<<1, 64, 0, s>>>(dst, v);
+  HPC_LAUNCH_CHECK("put_kernel");
+  return HPC_OK;
+}
+
 // The device instance table from the host bookkeeping and the current buffers.
 hpc_status write_inst_table(hpc_ctx *c) {
   std::vector<Inst> t((size_t)c->count);
@@ -208,8 +227,13 @@ hpc_status write_inst_table(hpc_ctx *c) {
   ++c->snap_epoch;
   for (auto &I : t) I.snap_epoch = c->snap_epoch;
   c->inst_host = t;
-  HPC_CUDA(cudaMemcpyAsync(c->inst, c->inst_host.data(), sizeof(Inst) * t.size(), cudaMemcpyHostToDevice, c->stream));
-  HPC_CUDA(cudaStreamSynchronize(c->stream));
+  if (c->count == 1) {
+    const hpc_status s = put(c->inst, c->inst_host[0], c->stream);
+    if (s != HPC_OK) return s;
+  } else {
+    HPC_CUDA(cudaMemcpyAsync(c->inst, c->inst_host.data(), sizeof(Inst) * t.size(), cudaMemcpyHostToDevice, c->stream));
+    HPC_CUDA(cudaStreamSynchronize(c->stream));
+  }
   ++c->inst_version;
   return HPC_OK;
 }
@@ -295,6 +319,8 @@ hpc_status enqueue_level(hpc_ctx *c, int level, bool timed) {
   hpc_status s;
   const Launch L = make_launch(c, level);
   cudaEvent_t *ev = c->evl[level];
+  for (int q = 0; timed && q < 4; ++q)  // made when the level is first timed: most contexts run few levels
+    if (!ev[q]) HPC_CUDA(cudaEventCreate(&ev[q]));
   const bool queue = !c->cor64_valid;  // FP64 re-tests deferred to the re-test kernel
   if (timed) HPC_CUDA(cudaEventRecord(ev[0], c->stream));
   if (level == 0) {
@@ -686,6 +712,12 @@ hpc_status ensure_meta(hpc_ctx *c) {
   hpc_status s;
   if ((s = dev_alloc(&c->meta, (int64_t)m.size(), "correlation metadata")) != HPC_OK) return s;
   if ((s = dev_alloc(&c->meta_denom, C, "correlation metadata")) != HPC_OK) return s;
+  if (C == 1) {
+    Words<14> w;  // 11 C + 3
+    std::copy(m.begin(), m.end(), w.w);
+    if ((s = put((Words<14> *)c->meta, w, c->stream)) != HPC_OK) return s;
+    return put(c->meta_denom, den[0], c->stream);
+  }
   HPC_CUDA(cudaMemcpyAsync(c->meta, m.data(), sizeof(long long) * m.size(), cudaMemcpyHostToDevice, c->stream));
   HPC_CUDA(cudaMemcpyAsync(c->meta_denom, den.data(), sizeof(double) * den.size(), cudaMemcpyHostToDevice, c->stream));
   HPC_CUDA(cudaStreamSynchronize(c->stream));
@@ -808,10 +840,14 @@ hpc_status correlation_device(hpc_ctx *c, const void *X, bool f32) {
             HPC_OK)
           return s;
       }
-      if ((s = dev_alloc(&c->tc_maps, 2 * c->count, "tensor maps")) != HPC_OK) return s;
-      HPC_CUDA(cudaMemcpyAsync(c->tc_maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice,
-                               c->stream));
-      HPC_CUDA(cudaStreamSynchronize(c->stream));
+      if (c->count == 1) {
+        std::copy(maps.begin(), maps.end(), c->own_maps);  // travel with the launch
+      } else {
+        if ((s = dev_alloc(&c->tc_maps, 2 * c->count, "tensor maps")) != HPC_OK) return s;
+        HPC_CUDA(cudaMemcpyAsync(c->tc_maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice,
+                                 c->stream));
+        HPC_CUDA(cudaStreamSynchronize(c->stream));
+      }
     }
     if ((s = launch_standardise(X, f32, sa, sa.count ? c->total_rows : 0, pair ? nullptr : c->Z,
                                 pair ? c->zpair : nullptr, ztot, c->tcP, c->stream)) != HPC_OK)
@@ -823,6 +859,7 @@ hpc_status correlation_device(hpc_ctx *c, const void *X, bool f32) {
     ta.count = c->count;
     ta.tile_prefix = gram_args(c).p + c->count;
     ta.maps = c->tc_maps;
+    std::copy(c->own_maps, c->own_maps + 2, ta.own);
     ta.c_off = gram_args(c).c_off;
     ta.p = gram_args(c).p;
     ta.n = sa.n;
@@ -917,7 +954,7 @@ hpc_status load_correlation(hpc_ctx *c, const double *C, cudaMemcpyKind kind) {
 }
 
 hpc_status create(hpc_ctx **out, int count, const int64_t *p, const int64_t *n, const double *alpha,
-                  const hpc_opts *opts);
+                  const hpc_opts *opts, cudaStream_t stream = nullptr);
 
 }  // namespace
 
@@ -960,6 +997,9 @@ int wide1_cols(const WideShape *sh, int count) {
 }
 
 // for the server's shared launches (serve.cu)
+hpc_status ctx_create_on(hpc_ctx **out, int64_t p, int64_t n, const hpc_opts *opts, cudaStream_t stream) {
+  return create(out, 1, &p, &n, nullptr, opts, stream);
+}
 hpc_status ctx_size_after_level0(hpc_ctx *c) {
   bool changed = false;
   return ensure_capacity(c, &changed);
@@ -1070,27 +1110,16 @@ hpc_status hpc_ctx_destroy(hpc_ctx *c) {
     dev_free(xs);
     c->X_stage = nullptr;
   }
-  dev_free(c->adj);
+  dev_free(c->fixed);
   dev_free(c->adj0);
   dev_free(c->wide_items);
   dev_free(c->wide_scratch);
   dev_free(c->adj_bytes);
-  dev_free(c->deg);
-  dev_free(c->rowptr);
-  dev_free(c->row_work);
-  dev_free(c->row_dirty);
   dev_free(c->colidx);
   dev_free(c->recs);
   dev_free(c->rq);
   dev_free(c->rq_val);
   dev_free(c->rq_done);
-  dev_free(c->ctr);
-  dev_free(c->gctr);
-  dev_free(c->lc);
-  dev_free(c->inst);
-  dev_free(c->prefixes);
-  dev_free(c->work_prefix);
-  dev_free(c->seg);
   dev_free(c->meta);
   dev_free(c->meta_denom);
   dev_free(c->tune_dev);
@@ -1127,6 +1156,7 @@ hpc_status hpc_ctx_set_stream(hpc_ctx *c, void *stream) {
   hpc_status s = check_ctx(c);
   if (s != HPC_OK) return s;
   HPC_CUDA(cudaStreamSynchronize(c->stream));
+  if (!stream && !c->own_stream) HPC_CUDA(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));
   c->stream = stream ? (cudaStream_t)stream : c->own_stream;
   return HPC_OK;
 }
@@ -1949,7 +1979,7 @@ namespace hpc {
 namespace {
 
 hpc_status create(hpc_ctx **out, int count, const int64_t *p, const int64_t *n, const double *alpha,
-                  const hpc_opts *opts) {
+                  const hpc_opts *opts, cudaStream_t stream) {
   if (!out) {
     set_error("null output pointer");
     return HPC_ERR_INVALID_ARG;
@@ -2061,14 +2091,13 @@ hpc_status create(hpc_ctx **out, int count, const int64_t *p, const int64_t *n, 
   bool ev_ok = true;
   for (auto &ev : c->evc) ev_ok = ev_ok && cudaEventCreate(&ev) == cudaSuccess;
   for (auto &ev : c->evr) ev_ok = ev_ok && cudaEventCreate(&ev) == cudaSuccess;
-  for (auto &lv : c->evl)
-    for (auto &ev : lv) ev_ok = ev_ok && cudaEventCreate(&ev) == cudaSuccess;
-  if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess || !ev_ok) {
+  if (stream) c->stream = stream;
+  else if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) == cudaSuccess) c->stream = c->own_stream;
+  if (!c->stream || !ev_ok) {
     cudaGetLastError();
     set_error("stream/event creation failed");
     return fail(HPC_ERR_CUDA);
   }
-  c->stream = c->own_stream;
   // grids of the levels this context can run (up to its max_level): a context that stays
   // at low levels never loads the level-17..32 kernel, whose local-memory stack frame
   // (35 KB per thread) would otherwise be reserved for the whole device
@@ -2087,22 +2116,38 @@ hpc_status create(hpc_ctx **out, int count, const int64_t *p, const int64_t *n, 
   if (c->rec_ids > 16) retest_setup();  // the re-test kernel of levels 17-32
   if (o.precision != HPC_PREC_MIXED_TC && (s = dev_alloc(&c->cor64, cor, "cor64")) != HPC_OK) return fail(s);
   if (o.precision != HPC_PREC_FP64 && (s = dev_alloc(&c->cor32, cor, "cor32")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->adj, adj, "adjacency")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->deg, rows, "degrees")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->rowptr, rows, "row offsets")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->row_work, rows, "row work")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->row_dirty, rows, "stale-row marks")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->ctr, (int64_t)count * kLevels, "level counters")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->gctr, count, "counters")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->lc, kLevels, "launch counters")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->inst, count, "instance table")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->prefixes, (int64_t)pre.size(), "prefixes")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->work_prefix, (int64_t)kLevels * (count + 1), "work prefixes")) != HPC_OK) return fail(s);
-  if ((s = dev_alloc(&c->seg, (int64_t)kLevels * segs, "segment sums")) != HPC_OK) return fail(s);
+  // the small arrays in one allocation, each on a 256-byte boundary
+  {
+    int64_t at = 0;
+    std::vector<std::pair<void **, int64_t>> parts;
+    auto part = [&](auto **ptr, int64_t n) {
+      parts.emplace_back((void **)ptr, at);
+      at += ((int64_t)sizeof(**ptr) * n + 255) / 256 * 256;
+    };
+    part(&c->adj, adj);
+    part(&c->deg, rows);
+    part(&c->rowptr, rows);
+    part(&c->row_work, rows);
+    part(&c->row_dirty, rows);
+    part(&c->ctr, (int64_t)count * kLevels);
+    part(&c->gctr, count);
+    part(&c->lc, kLevels);
+    part(&c->inst, count);
+    part(&c->prefixes, (int64_t)pre.size());
+    part(&c->work_prefix, (int64_t)kLevels * (count + 1));
+    part(&c->seg, (int64_t)kLevels * segs);
+    if ((s = dev_alloc(&c->fixed, at, "context state")) != HPC_OK) return fail(s);
+    for (auto &q : parts) *q.first = c->fixed + q.second;
+  }
   c->ctr_host = new DevCounters[(size_t)count * kLevels];
   c->gctr_host = new DevGlobal[(size_t)count];
-  if (cudaMemcpyAsync(c->prefixes, pre.data(), sizeof(long long) * pre.size(), cudaMemcpyHostToDevice, c->stream) !=
-          cudaSuccess ||
+  if (count == 1) {
+    Words<8> w;  // 4 (count + 1)
+    std::copy(pre.begin(), pre.end(), w.w);
+    if ((s = put((Words<8> *)c->prefixes, w, c->stream)) != HPC_OK) return fail(s);
+  }
+  if ((count > 1 && cudaMemcpyAsync(c->prefixes, pre.data(), sizeof(long long) * pre.size(), cudaMemcpyHostToDevice,
+                                    c->stream) != cudaSuccess) ||
       cudaMemsetAsync(c->ctr, 0, sizeof(DevCounters) * (size_t)count * kLevels, c->stream) != cudaSuccess ||
       cudaMemsetAsync(c->gctr, 0, sizeof(DevGlobal) * (size_t)count, c->stream) != cudaSuccess ||
       cudaMemsetAsync(c->lc, 0, sizeof(LaunchCounters) * kLevels, c->stream) != cudaSuccess) {

@@ -88,7 +88,7 @@ __device__ __forceinline__ void fail(TcSmem &sm, int *err) {
 }
 
 __global__ void __launch_bounds__(kThreadsTc, 1)
-    gram_tc_kernel(float *__restrict__ Call, TcArgs ta) {
+    gram_tc_kernel(float *__restrict__ Call, const __grid_constant__ TcArgs ta) {
   extern __shared__ uint8_t smem_raw[];
   TcSmem &sm = *reinterpret_cast<TcSmem *>((((uintptr_t)smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
   const int kbq = (int)((ta.n[inst] + TK - 1) / TK);  // k-blocks per product
   const int64_t n_pad = (int64_t)kbq * TK;
   const int kblocks = kSlices * kbq;
-  const CUtensorMap *mapP = ta.maps + 2 * inst, *mapQ = ta.maps + 2 * inst + 1;
+  const CUtensorMap *mapP = ta.maps ? ta.maps + 2 * inst : ta.own, *mapQ = mapP + 1;
   float *__restrict__ C = Call + ta.c_off[inst];
   int *err = ta.err;
   // tiles in bands of kBand row blocks, each band column block by column block, so

@@ -387,7 +387,8 @@ hpc_status tc_make_maps(CUtensorMap *mp, CUtensorMap *mq, const __nv_bfloat16 *P
 struct TcArgs {                     // grouped tensor-core Gram
   int count;
   const long long *tile_prefix;     // 128 x 128 upper-triangle tiles (count + 1)
-  const CUtensorMap *maps;          // 2 per instance (P, Q), 64-byte aligned, device
+  const CUtensorMap *maps;          // 2 per instance (P, Q), 64-byte aligned, device; null: `own`
+  CUtensorMap own[2];               // the maps of a single instance, read from the parameter bank
   const long long *c_off, *p, *n;
   int *err;
 };
@@ -440,6 +441,8 @@ TuneEntry tune_get(int p_bucket, int level, int deg_bucket);  // by bucket indic
 // record buffers sized from its level-0 counters (ctr_host filled by the caller), and
 // the bytes of the re-test queue a context of sum p^2 would hold
 hpc_status ctx_size_after_level0(hpc_ctx *c);
+// a single-instance context on the caller's stream, without one of its own
+hpc_status ctx_create_on(hpc_ctx **out, int64_t p, int64_t n, const hpc_opts *opts, cudaStream_t stream);
 long long ctx_retest_queue_bytes(long long sum_p2);
 // entries of re-test scratch for a queue of `cap` items: three per item (a level-1
 // re-test), at most 32 Mi
@@ -486,6 +489,8 @@ struct hpc_ctx {
   int sm_count = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t own_stream = nullptr;  // the context's stream; `stream` may be a caller's
+  uint8_t *fixed = nullptr;       // one allocation for the small arrays of create()
+  CUtensorMap own_maps[2];        // the tensor maps of a single instance
   // packed device buffers
   double *cor64 = nullptr;        // sum p^2 (absent in tensor-core mode unless loaded)
   float *cor32 = nullptr;         // sum p^2 (mixed modes)

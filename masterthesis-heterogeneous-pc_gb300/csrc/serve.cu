@@ -147,9 +147,8 @@ hpc_status admit(hpc_server *sv, Request *r) {
   o.precision = sv->opts.precision;
   o.max_level = sv->opts.max_level;
   o.alpha = r->alpha;
-  hpc_status s = hpc_ctx_create(&r->ctx, r->p, r->n, &o);
+  hpc_status s = ctx_create_on(&r->ctx, r->p, r->n, &o, sv->st);
   if (s != HPC_OK) return s;
-  if ((s = hpc_ctx_set_stream(r->ctx, sv->st)) != HPC_OK) return s;
   if ((s = grow(&sv->stage, &sv->stage_cap, r->p * r->n, sv->st)) != HPC_OK) return s;
   HPC_CUDA(cudaMemcpyAsync(sv->stage, r->X, sizeof(float) * (size_t)(r->p * r->n), cudaMemcpyHostToDevice, sv->st));
   if ((s = hpc_correlation_device_f32(r->ctx, sv->stage)) != HPC_OK) return s;
