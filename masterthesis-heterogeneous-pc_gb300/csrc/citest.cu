@@ -101,13 +101,15 @@ __global__ void pack_records_kernel(const Inst *__restrict__ inst, const RecSegm
   }
 }
 
-__device__ __forceinline__ double warp_dot(const Inst &I, int64_t a, int64_t b) {
+// samples [k0, end) of the product of two standardised columns
+__device__ __forceinline__ double warp_dot(const Inst &I, int64_t a, int64_t b, int64_t k0, int64_t end) {
   const int lane = threadIdx.x & 31;
-  double s = zdot(I, a, b, lane, 32);
+  double s = zdot(I, a, b, k0 + lane, 32, end);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
 }
+__device__ __forceinline__ double warp_dot(const Inst &I, int64_t a, int64_t b) { return warp_dot(I, a, b, 0, I.n_z); }
 
 // FP64 re-tests deferred by the level kernels (instances without an FP64 matrix). A
 // re-test of level l needs the E = (l + 2)(l + 1) / 2 FP64 correlation entries among
@@ -121,9 +123,13 @@ __device__ __forceinline__ double warp_dot(const Inst &I, int64_t a, int64_t b) 
 // scratch take a warp each. Level-0 items (one entry) set the kept bits of both
 // triangles; level >= 1 items remove the edge. The done counters return to zero when
 // their item is evaluated, ready for the next launch.
+// With few items the samples of a dot product are cut into up to kRetestParts parts of a warp each
+// (a warp alone goes over 8000 samples in about 20 us, and most levels of a deep skeleton have a
+// handful of re-tests): the warp completing the item adds up the parts, in their order.
 // KM: the highest level of the launch's items (16 for levels up to 16, HPC_MAX_LEVEL
 // above), which sizes the FP64 fallback's local arrays.
 constexpr int kRetestWarps = 8;
+constexpr int kRetestParts = 8;
 
 // the variable at position r of a re-test's matrix order (i, j, S)
 __device__ __forceinline__ int64_t retest_var(const RetestItem *it, int r) {
@@ -140,14 +146,82 @@ __device__ __forceinline__ void entry_rc(int e, int k, int &r, int &c) {
   c = r + 1 + e;
 }
 
-// lane 0: the FP64 decision of item it from its matrix M (k x k, warp-filled)
+// partial_r_of_matrix by the whole warp, M in shared memory (left as it was where *ok is false, which
+// is where it takes the pseudoinverse): a lane per member, column by column of the factor, every
+// entry in the same operations and order -- so the same value. One lane alone steps through
+// l^3 / 6 dependent FP64 operations, about 80 us at level 12, longer than all the dot products
+// of a level with a few re-tests. The factor goes to the lower triangle of the S block, w_i and
+// w_j to the first two columns; the upper triangle keeps the entries.
+__device__ __forceinline__ double warp_partial_r(double *M, int l, bool *nan_p, bool *ok) {
+  const int lane = threadIdx.x & 31, k = l + 2;
+  bool bad = false;
+  for (int q = lane; q < k * k; q += 32) bad |= isnan(M[q]);
+  *nan_p = __any_sync(0xffffffffu, bad);
+  *ok = true;
+  if (*nan_p) return 0.0;
+  double *row = M + (lane + 2) * k;  // lane < l: its member's row
+  double d = 1.0, vx = lane < l ? M[lane + 2] : 0.0, vy = lane < l ? M[k + lane + 2] : 0.0;
+  for (int c = 0; c < l; ++c) {
+    if (!__shfl_sync(0xffffffffu, d > 1e-10, c)) {
+      *ok = false;
+      break;
+    }
+    if (lane == c) {
+      const double lcc = sqrt(d);
+      row[c + 2] = lcc;
+      row[0] = vx / lcc;
+      row[1] = vy / lcc;
+    }
+    __syncwarp();
+    if (lane > c && lane < l) {
+      const double *rc = M + (c + 2) * k;
+      double v = rc[lane + 2];
+      for (int q = 0; q < c; ++q) v -= row[q + 2] * rc[q + 2];
+      v /= rc[c + 2];
+      row[c + 2] = v;
+      d -= v * v;
+      vx -= v * rc[0];
+      vy -= v * rc[1];
+    }
+    __syncwarp();
+  }
+  double r = 0.0;
+  if (*ok) {
+    double ax = 1.0, ay = 1.0, b = M[1];
+    for (int q = 0; q < l; ++q) {
+      const double wx = M[(q + 2) * k], wy = M[(q + 2) * k + 1];
+      ax -= wx * wx;
+      ay -= wy * wy;
+      b -= wx * wy;
+    }
+    *ok = ax > 1e-10 && ay > 1e-10;
+    r = b / sqrt(ax * ay);
+  }
+  if (!*ok) {  // the matrix as it was
+    __syncwarp();
+    for (int q = lane; q < k * k; q += 32) {
+      const int a = q / k, c = q - a * k;
+      if (a > c) M[q] = M[c * k + a];
+      if (a == c) M[q] = 1.0;
+    }
+    __syncwarp();
+  }
+  return r;
+}
+
+// The FP64 decision of item it from its matrix M (k x k, warp-filled); whole warp.
 template <int KM>
 __device__ __forceinline__ void retest_decide(const Launch &L, const Inst &I, const RetestItem *it, int l, double *M) {
-  bool nan_p;
-  const double r = partial_r_of_matrix<KM>(M, l, &nan_p);
-  double pv;
-  const int64_t i = it->i, j = it->j;
-  if (decide_of_r(I, r, nan_p, &pv) && claim_edge(I, i, j)) write_record(I, L.level, i, j, it->ids, l, pv);
+  const int lane = threadIdx.x & 31;
+  bool nan_p = false, ok = false;
+  double r = 0.0;
+  if (l > 1) r = warp_partial_r(M, l, &nan_p, &ok);
+  if (lane == 0) {
+    if (!ok) r = partial_r_of_matrix<KM>(M, l, &nan_p);
+    double pv;
+    const int64_t i = it->i, j = it->j;
+    if (decide_of_r(I, r, nan_p, &pv) && claim_edge(I, i, j)) write_record(I, L.level, i, j, it->ids, l, pv);
+  }
 }
 
 // Levels 1-4 (K = l + 2 <= 6 variables): one warp per item, every lane accumulating the
@@ -329,7 +403,12 @@ __global__ void __launch_bounds__(kRetestWarps * 32, 2) retest_kernel(const __gr
     }
     return;
   }
-  if (l <= kColumnTop) {
+  const unsigned long long E = (unsigned long long)(k * (k - 1) / 2);
+  // by columns once the items' entries would keep every warp busy: an item's columns take a warp
+  // three (level 1) to eight (level 4) times as long as one entry does (30 items of level 4 in a batch
+  // of 24: 134 us by columns, 34 us by entries in parts)
+  const bool by_columns = l <= kColumnTop && count * E > nwarps;
+  if (by_columns) {
     // an item per warp from its columns (instances with FP32-pair data; FP64 Z takes
     // the general path below)
     for (unsigned long long q = warp; q < count; q += nwarps) {
@@ -343,19 +422,21 @@ __global__ void __launch_bounds__(kRetestWarps * 32, 2) retest_kernel(const __gr
         default: retest_item_columns<6>(I, it, M); break;
       }
       __syncwarp();
-      if (lane == 0) retest_decide<KM>(L, I, it, l, M);
+      retest_decide<KM>(L, I, it, l, M);
       __syncwarp();
     }
   }
-  const int E = k * (k - 1) / 2;
   // the items not taken above run entry by entry (the first W of them) or a warp each
-  const bool by_columns = l <= kColumnTop;
-  const unsigned long long W =
-      L.rq_val ? min(count, (unsigned long long)(L.rq_vcap / E)) : 0ull;
-  const unsigned long long units = W * (unsigned long long)E;
+  int parts = 1;
+  while (L.rq_val && parts < kRetestParts && count * E * (unsigned)parts * 2 <= nwarps &&
+         count * E * (unsigned)parts * 2 <= (unsigned long long)L.rq_vcap)
+    parts *= 2;
+  const unsigned long long EP = E * (unsigned)parts;  // scratch entries of an item
+  const unsigned long long W = L.rq_val ? min(count, (unsigned long long)L.rq_vcap / EP) : 0ull;
+  const unsigned long long units = W * EP;
   for (unsigned long long u = warp; u < units; u += nwarps) {
-    const unsigned long long q = u / (unsigned long long)E;
-    const int e = (int)(u - q * (unsigned long long)E);
+    const unsigned long long q = u / EP;
+    const int x = (int)(u - q * EP), e = x / parts, part = x - e * parts;
     const RetestItem *it = L.rq + q;
     const Inst &I = *inst_of(L, it->inst);
     if (by_columns && I.zh) continue;  // decided above
@@ -365,16 +446,18 @@ __global__ void __launch_bounds__(kRetestWarps * 32, 2) retest_kernel(const __gr
       entry_rc(e, k, r, c);
       const int64_t va = retest_var(it, r), vb = retest_var(it, c);
       double v;
-      if (!ecache_get(I, va, vb, &v)) {
+      if (parts > 1) {  // (the parts of an entry do not look at the store: it may change between them)
+        v = warp_dot(I, va, vb, I.n_z * part / parts, I.n_z * (part + 1) / parts);
+      } else if (!ecache_get(I, va, vb, &v)) {
         v = warp_dot(I, va, vb) / I.denom;
         if (lane == 0) ecache_put(I, va, vb, v);
       }
-      if (lane == 0) L.rq_val[q * (unsigned long long)E + e] = v;
+      if (lane == 0) L.rq_val[u] = v;
     }
     unsigned last = 0;
     if (lane == 0) {
       __threadfence();
-      last = atomicAdd(L.rq_done + q, 1u) == (unsigned)(E - 1);
+      last = atomicAdd(L.rq_done + q, 1u) == (unsigned)(EP - 1);
     }
     if (!__shfl_sync(0xffffffffu, last, 0)) continue;
     // the item's last entry: gather its matrix and decide
@@ -387,12 +470,18 @@ __global__ void __launch_bounds__(kRetestWarps * 32, 2) retest_kernel(const __gr
       if (r != c) {
         const int a = r < c ? r : c, b2 = r < c ? c : r;
         const int eidx = a * k - a * (a + 1) / 2 + (b2 - a - 1);  // entry_rc's numbering
-        v = __ldcg(L.rq_val + q * (unsigned long long)E + eidx);
+        const double *at = L.rq_val + q * EP + (unsigned)(eidx * parts);
+        v = __ldcg(at);
+        if (parts > 1) {
+          for (int s = 1; s < parts; ++s) v += __ldcg(at + s);
+          v /= I.denom;
+          if (r < c) ecache_put(I, retest_var(it, r), retest_var(it, c), v);
+        }
       }
       M[t] = v;
     }
     __syncwarp();
-    if (lane == 0) retest_decide<KM>(L, I, it, l, M);
+    retest_decide<KM>(L, I, it, l, M);
     __syncwarp();
   }
   // items beyond the scratch: a warp each
@@ -414,7 +503,7 @@ __global__ void __launch_bounds__(kRetestWarps * 32, 2) retest_kernel(const __gr
       }
     }
     __syncwarp();
-    if (lane == 0) retest_decide<KM>(L, I, it, l, M);
+    retest_decide<KM>(L, I, it, l, M);
     __syncwarp();
   }
 }

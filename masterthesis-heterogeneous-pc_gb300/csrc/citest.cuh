@@ -75,7 +75,7 @@ __device__ __forceinline__ double exact_entry(const Inst &I, int64_t x, int64_t 
   if (I.cor64) return I.cor64[x * I.p + y];
   double v;
   if (ecache_get(I, x, y, &v)) return v;
-  v = zdot(I, x, y, 0, 1) / I.denom;
+  v = zdot(I, x, y, 0, 1, I.n_z) / I.denom;
   ecache_put(I, x, y, v);
   return v;
 }

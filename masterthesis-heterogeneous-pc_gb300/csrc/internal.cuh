@@ -240,17 +240,17 @@ __device__ __forceinline__ void ecache_put(const Inst &I, int64_t a, int64_t b, 
   atomicOr(I.ev + (bit >> 5), 1u << (bit & 31));
 }
 
-// Sum over samples k = k0, k0 + step, ... < n of z_a[k] * z_b[k], the FP64-standardised
-// variables a and b of one instance. From Z: FP64 FMAs. From the FP32 pairs: each
+// Sum over samples k = k0, k0 + step, ... < end of z_a[k] * z_b[k], the FP64-standardised
+// variables a and b of one instance (end at most its n_z). From Z: FP64 FMAs. From the FP32 pairs: each
 // product zh_a zh_b with its exact rounding error (fmaf) and the cross terms, summed
 // with compensation (TwoSum) in FP32 and carried into FP64 every 16 samples -- about
 // 2^-45 relative per block, and FP32 arithmetic instead of this GPU's 1/64-rate FP64.
-__device__ __forceinline__ double zdot(const Inst &I, int64_t a, int64_t b, int64_t k0, int64_t step) {
+__device__ __forceinline__ double zdot(const Inst &I, int64_t a, int64_t b, int64_t k0, int64_t step, int64_t end) {
   const int64_t n = I.n_z;
   double s = 0.0;
   if (I.Z) {
     const double *x = I.Z + a * n, *y = I.Z + b * n;
-    for (int64_t k = k0; k < n; k += step) s = fma(x[k], y[k], s);
+    for (int64_t k = k0; k < end; k += step) s = fma(x[k], y[k], s);
     return s;
   }
   const float *xh = I.zh + a * n, *xl = I.zl + a * n, *yh = I.zh + b * n, *yl = I.zl + b * n;
@@ -268,14 +268,14 @@ __device__ __forceinline__ double zdot(const Inst &I, int64_t a, int64_t b, int6
   int64_t k = k0;
   // full blocks: no bounds test inside, so that all 64 loads of a block issue before the
   // arithmetic that waits for them
-  for (; k + 15 * step < n; k += 16 * step) {
+  for (; k + 15 * step < end; k += 16 * step) {
     float sh = 0.f, sl = 0.f;
 #pragma unroll
     for (int u = 0; u < 16; ++u) add(k + u * step, sh, sl);
     s += (double)sh + (double)sl;
   }
   float sh = 0.f, sl = 0.f;
-  for (; k < n; k += step) add(k, sh, sl);
+  for (; k < end; k += step) add(k, sh, sl);
   return s + ((double)sh + (double)sl);
 }
 
