@@ -552,11 +552,11 @@ void *kernel_for(int level, int l1_variant) {
   }
 }
 
-// dynamic shared memory of a level kernel: the row-offset cache of levels >= 2, the chunk of
-// the wide level-1 body
-int level_smem(int level, int variant) {
+// dynamic shared memory of a level kernel: the row offsets of own_scan (`rows` of them; none at
+// level 1), the chunk of the wide level-1 body
+int level_smem(int level, int variant, int rows) {
   if (level == 1) return (variant & kWide) ? (int)sizeof(Wide1Smem) : 0;
-  return kRowCache * (int)sizeof(unsigned long long);
+  return rows * (int)sizeof(unsigned long long);
 }
 
 }  // namespace
@@ -572,7 +572,7 @@ int citest_grid(int precision, int level, int device, int l1_variant) {
   if (slot)
     if (const int g = slot->load(std::memory_order_acquire)) return g;
   void *k = mixed ? kernel_for<true>(level, l1_variant) : kernel_for<false>(level, l1_variant);
-  const int smem = level_smem(level, l1_variant);
+  const int smem = level_smem(level, l1_variant, kRowCache);  // the most it may have
   // beyond the default 48 KB of shared memory
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) cudaGetLastError();
   int per_sm = 0, sms = 0;
@@ -636,6 +636,7 @@ hpc_status launch_level(const Launch &L, int precision, int grid, int l1_variant
   void *k = precision == HPC_PREC_FP64 ? kernel_for<false>(L.level, l1_variant)
                                        : kernel_for<true>(L.level, l1_variant);
   Launch args = L;
+  if (l1_variant != kSetOrder && (l1_variant & kWide)) args.row_cache = 0;  // the wide-row kernels scan together
   void *params[] = {&args};
   // cooperative: every block co-resident, as the grid barriers require
   cudaLaunchAttribute attr[1];
@@ -644,7 +645,7 @@ hpc_status launch_level(const Launch &L, int precision, int grid, int l1_variant
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = L.level > 1 && !L.row_cache ? 0 : (size_t)level_smem(L.level, l1_variant);
+  cfg.dynamicSmemBytes = (size_t)level_smem(L.level, l1_variant, args.row_cache ? (int)L.inst0.p + 1 : 0);
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;

@@ -511,17 +511,18 @@ __device__ __forceinline__ int64_t find_row_from(const unsigned long long *row_w
   return lo;
 }
 
-// The row offsets of a single-instance level copied into shared memory by the whole
-// block (one round of coalesced loads), so that every row search of the CI tests
-// stays on the SM; null when the launch has no cache (several instances, or more than
-// kRowCache - 1 rows: the shared memory is then left to the L1 cache).
-__device__ __forceinline__ const unsigned long long *cache_row_work(const Launch &L, unsigned long long *smem) {
-  if (!smem || !L.row_cache) return nullptr;
-  const Inst &I = *inst_of(L, 0);
-  for (int64_t r = threadIdx.x; r <= I.p; r += blockDim.x) smem[r] = __ldcg(I.row_work + r);
-  __syncthreads();
-  return smem;
-}
+// The flattened index of a level's units: their number and each row's offset -- of a single
+// instance of up to kRowCache - 1 rows formed by every block for itself (own_scan: `own`, in shared
+// memory), else from the scan phase (work_prefix and the instances' row_work).
+struct Work {
+  unsigned long long total;
+  const unsigned long long *own, *prefix;
+  int count;
+  __device__ __forceinline__ const unsigned long long *rows(const Inst &I) const { return own ? own : I.row_work; }
+  __device__ __forceinline__ int inst(unsigned long long t) const { return find_inst_u(prefix, count, t); }
+  __device__ __forceinline__ unsigned long long begin(int b) const { return own ? 0ull : prefix[b]; }
+  __device__ __forceinline__ unsigned long long end(int b) const { return own ? total : prefix[b + 1]; }
+};
 
 // Row of a warp-uniform position t: a 32-ary search (coalesced probes, two or three
 // rounds for thousands of rows) instead of log2(p) dependent loads. Whole warp.
@@ -690,12 +691,10 @@ __device__ __forceinline__ bool push_retest(const Launch &L, int b, int64_t i, i
 }
 
 // The level's tile policy: the forced one, else the context's table entry for (largest
-// p, level, largest degree at the level start), else the defaults. Read after the
-// scan phase's grid barrier (the degree is formed there).
-__device__ __forceinline__ TuneEntry tile_policy(const Launch &L) {
+// p, level, largest degree md at the level start), else the defaults.
+__device__ __forceinline__ TuneEntry tile_policy(const Launch &L, int md) {
   TuneEntry te = L.force;
   if (te.tile_cap <= 0 && L.tune) {
-    const int md = *(volatile const int *)&L.lc->max_deg;
     te = L.tune[((size_t)L.p_bucket * (HPC_MAX_LEVEL + 1) + L.level) * kTuneDB + tune_bucket(md, kTuneDB)];
   }
   if (te.tile_cap <= 0) te = TuneEntry{kTuneDefaultCap, kTuneDefaultTpl, kTuneDefaultEdgeLanes, 0};
@@ -740,7 +739,7 @@ struct alignas(16) TestSmem {
 };
 
 template <int LT, bool MIXED>
-__device__ __forceinline__ void tests_generic(const Launch &L, unsigned long long *rw_smem, const TuneEntry &te,
+__device__ __forceinline__ void tests_generic(const Launch &L, const Work &wk, const TuneEntry &te,
                                               TestSmem<LT, MIXED> &sm) {
   constexpr int LA = LT > 0 ? LT : HPC_MAX_LEVEL;
   const int l = LT > 0 ? LT : L.level;
@@ -755,9 +754,8 @@ __device__ __forceinline__ void tests_generic(const Launch &L, unsigned long lon
   int *np = sm.np + wib;
   if (lane == 0) *np = 0;
   __syncwarp();
-  const unsigned long long total = L.work_prefix[L.count];
+  const unsigned long long total = wk.total;
   if (total == 0) return;
-  const unsigned long long *rw_c = cache_row_work(L, rw_smem);
   const unsigned long long lanes = (unsigned long long)gridDim.x * blockDim.x;
   const int m = tile_tests_per_lane(total, lanes, te, true);
   const unsigned long long per_tile = 32ull * (unsigned long long)m;
@@ -780,11 +778,13 @@ __device__ __forceinline__ void tests_generic(const Launch &L, unsigned long lon
     unsigned executed = 0, retests = 0;
     int b_last = -1;
     // instance and row of the tile start (whole warp), then each lane's row
-    int b = find_inst_u(L.work_prefix, L.count, t0);
+    int b = wk.inst(t0);
     const Inst *I = inst_of(L, b);
-    unsigned long long base_t = L.work_prefix[b];
-    const int64_t i0 = warp_find_row(rw_c ? rw_c : I->row_work, I->p, t0 - base_t);
-    if (kBlk && (i0 != blk_i || b != blk_b)) {  // the block of the tile's first row
+    unsigned long long base_t = wk.begin(b);
+    const int64_t i0 = warp_find_row(wk.rows(*I), I->p, t0 - base_t);
+    // the block of the tile's first row, where its lanes have tests enough to be worth the copy
+    // (three round trips to memory, as long as two tests from the matrix)
+    if (kBlk && m > 2 && (i0 != blk_i || b != blk_b)) {
       const int d0 = I->deg[i0];
       if (d0 <= kBlkD) {
         stage_block(*I, i0, d0, blk);
@@ -793,27 +793,35 @@ __device__ __forceinline__ void tests_generic(const Launch &L, unsigned long lon
       }
     }
     const bool active = t < tend;
-    const bool same = t < L.work_prefix[b + 1];
-    int64_t i = lane_find_row(rw_c ? rw_c : I->row_work, I->p, i0, (active && same ? t : t0) - base_t, active && same);
+    const bool same = t < wk.end(b);
+    int64_t i = lane_find_row(wk.rows(*I), I->p, i0, (active && same ? t : t0) - base_t, active && same);
     if (active && !same) {  // the tile runs into the next instance
-      b = find_inst_u(L.work_prefix, L.count, t);
+      b = wk.inst(t);
       I = inst_of(L, b);
-      base_t = L.work_prefix[b];
-      i = find_row(rw_c ? rw_c : I->row_work, I->p, t - base_t);
+      base_t = wk.begin(b);
+      i = find_row(wk.rows(*I), I->p, t - base_t);
     }
     if (active) {
       int d = I->deg[i];
       unsigned long long c = binom_fast(d - 1, l);
-      const unsigned long long off = t - base_t - (rw_c ? rw_c : I->row_work)[i];
+      const unsigned long long off = t - base_t - wk.rows(*I)[i];
       int s = (int)(off / c);
       unsigned long long rank = off - (unsigned long long)s * c;
       int base = I->rowptr[i];
       int64_t j = I->colidx[base + s];
-      bool alive = live_bit(I->adj, I->W, i, j);
       // a removed edge needs no subset: its rest is skipped below, and when the whole
-      // tile lies inside it, so are the edge's further tiles
-      if (alive) unrank_lex_fast(rank, l, d - 1, pos);
-      else if (lane == 0) skip_tiles_of_edge(L, t - rank + c, t0 + per_tile, per_tile, nwarps);
+      // tile lies inside it, so are the edge's further tiles (with a test or two a lane the subset
+      // is unranked while the live bit is on its way)
+      bool alive;
+      if (m <= 2) {
+        const uint32_t word = *(const volatile uint32_t *)(I->adj + i * I->W + (j >> 5));
+        unrank_lex_fast(rank, l, d - 1, pos);
+        alive = (word >> (j & 31)) & 1u;
+      } else {
+        alive = live_bit(I->adj, I->W, i, j);
+        if (alive) unrank_lex_fast(rank, l, d - 1, pos);
+      }
+      if (!alive && lane == 0) skip_tiles_of_edge(L, t - rank + c, t0 + per_tile, per_tile, nwarps);
       unsigned tested_edge = 0;
       int ci = 0;  // lowest position changed since the last test (rows below are valid)
       Fact<LA> F;
@@ -866,13 +874,13 @@ __device__ __forceinline__ void tests_generic(const Launch &L, unsigned long lon
           rank = 0;
           if (++s == d) {
             // next row with tests, possibly of the next instance
-            if (t >= L.work_prefix[b + 1]) {
-              b = find_inst_u(L.work_prefix, L.count, t);
+            if (t >= wk.end(b)) {
+              b = wk.inst(t);
               I = inst_of(L, b);
-              base_t = L.work_prefix[b];
-              i = find_row(rw_c ? rw_c : I->row_work, I->p, t - base_t);
+              base_t = wk.begin(b);
+              i = find_row(wk.rows(*I), I->p, t - base_t);
             } else {
-              i = find_row_from(rw_c ? rw_c : I->row_work, I->p, i, t - base_t);
+              i = find_row_from(wk.rows(*I), I->p, i, t - base_t);
             }
             d = I->deg[i];
             c = binom_fast(d - 1, l);
@@ -918,7 +926,7 @@ __device__ __forceinline__ void tests_generic(const Launch &L, unsigned long lon
 // rerun as in the set order -- the kernel then holds no inline FP64 re-test, whose
 // registers the interleaved body would otherwise spill for.
 template <bool MIXED, bool PF, bool QO = false>
-__device__ __forceinline__ void tests_l1(const Launch &L, unsigned long long *rw_smem, const TuneEntry &te) {
+__device__ __forceinline__ void tests_l1(const Launch &L, const Work &wk, const TuneEntry &te) {
   const int level = 1;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   __shared__ PendRem<1> s_pend[kThreads / 32][kPend];
@@ -927,9 +935,8 @@ __device__ __forceinline__ void tests_l1(const Launch &L, unsigned long long *rw
   int *np = s_np + wib;
   if (lane == 0) *np = 0;
   __syncwarp();
-  const unsigned long long total = L.work_prefix[L.count];
+  const unsigned long long total = wk.total;
   if (total == 0) return;
-  const unsigned long long *rw_c = cache_row_work(L, rw_smem);
   const unsigned long long lanes = (unsigned long long)gridDim.x * blockDim.x;
   const int m = tile_tests_per_lane(total, lanes, te, false);
   const unsigned long long per_tile = 32ull * (unsigned long long)m;
@@ -951,23 +958,23 @@ __device__ __forceinline__ void tests_l1(const Launch &L, unsigned long long *rw
     unsigned executed = 0, retests = 0;
     int b_last = -1;
     // instance and row of the tile start (whole warp), then each lane's row
-    int b = find_inst_u(L.work_prefix, L.count, t0);
+    int b = wk.inst(t0);
     const Inst *I = inst_of(L, b);
-    unsigned long long base_t = L.work_prefix[b];
-    const int64_t i0 = warp_find_row(rw_c ? rw_c : I->row_work, I->p, t0 - base_t);
+    unsigned long long base_t = wk.begin(b);
+    const int64_t i0 = warp_find_row(wk.rows(*I), I->p, t0 - base_t);
     const bool active = t < tend;
-    const bool same = t < L.work_prefix[b + 1];
-    int64_t i = lane_find_row(rw_c ? rw_c : I->row_work, I->p, i0, (active && same ? t : t0) - base_t, active && same);
+    const bool same = t < wk.end(b);
+    int64_t i = lane_find_row(wk.rows(*I), I->p, i0, (active && same ? t : t0) - base_t, active && same);
     if (active && !same) {  // the tile runs into the next instance
-      b = find_inst_u(L.work_prefix, L.count, t);
+      b = wk.inst(t);
       I = inst_of(L, b);
-      base_t = L.work_prefix[b];
-      i = find_row(rw_c ? rw_c : I->row_work, I->p, t - base_t);
+      base_t = wk.begin(b);
+      i = find_row(wk.rows(*I), I->p, t - base_t);
     }
     if (active) {
       int d = I->deg[i];
       int c = d - 1;  // tests per edge at level 1
-      unsigned long long off = t - base_t - (rw_c ? rw_c : I->row_work)[i];
+      unsigned long long off = t - base_t - wk.rows(*I)[i];
       int s = (int)(off / (unsigned long long)c);
       int rank = (int)(off - (unsigned long long)s * c);
       int base = I->rowptr[i];
@@ -1070,18 +1077,18 @@ __device__ __forceinline__ void tests_l1(const Launch &L, unsigned long long *rw
           rank -= c;
           moved = true;
           if (++s == d) {
-            if (t >= L.work_prefix[b + 1]) {
-              b = find_inst_u(L.work_prefix, L.count, t);
+            if (t >= wk.end(b)) {
+              b = wk.inst(t);
               I = inst_of(L, b);
-              base_t = L.work_prefix[b];
-              i = find_row(rw_c ? rw_c : I->row_work, I->p, t - base_t);
+              base_t = wk.begin(b);
+              i = find_row(wk.rows(*I), I->p, t - base_t);
             } else {
-              i = find_row_from(rw_c ? rw_c : I->row_work, I->p, i, t - base_t);
+              i = find_row_from(wk.rows(*I), I->p, i, t - base_t);
             }
             d = I->deg[i];
             c = d - 1;
             base = I->rowptr[i];
-            off = t - base_t - (rw_c ? rw_c : I->row_work)[i];
+            off = t - base_t - wk.rows(*I)[i];
             s = (int)(off / (unsigned long long)c);
             rank = (int)(off - (unsigned long long)s * c);
             break;
@@ -1277,7 +1284,7 @@ __device__ __forceinline__ uint64_t row_live_mask(const Inst &I, int64_t i, int 
 }
 
 template <int LT>
-__device__ __forceinline__ void tests_set(const Launch &L, unsigned long long *rw_smem, const TuneEntry &te,
+__device__ __forceinline__ void tests_set(const Launch &L, const Work &wk, const TuneEntry &te,
                                           TestSmem<LT, true> &sm) {
   constexpr int LA = LT;
   constexpr int l = LT;
@@ -1291,9 +1298,8 @@ __device__ __forceinline__ void tests_set(const Launch &L, unsigned long long *r
   int *np = sm.np + wib;
   if (lane == 0) *np = 0;
   __syncwarp();
-  const unsigned long long total = L.work_prefix[L.count];
+  const unsigned long long total = wk.total;
   if (total == 0) return;
-  const unsigned long long *rw_c = cache_row_work(L, rw_smem);
   const unsigned long long lanes = (unsigned long long)gridDim.x * blockDim.x;
   const int m = tile_tests_per_lane(total, lanes, te, true);
   const unsigned long long per_tile = 32ull * (unsigned long long)m;
@@ -1313,10 +1319,10 @@ __device__ __forceinline__ void tests_set(const Launch &L, unsigned long long *r
     const unsigned long long tend = min(t + (unsigned long long)m, total);
     unsigned executed = 0, retests = 0;
     int b_last = -1;
-    int b = find_inst_u(L.work_prefix, L.count, t0);
+    int b = wk.inst(t0);
     const Inst *I = inst_of(L, b);
-    unsigned long long base_t = L.work_prefix[b];
-    const int64_t i0 = warp_find_row(rw_c ? rw_c : I->row_work, I->p, t0 - base_t);
+    unsigned long long base_t = wk.begin(b);
+    const int64_t i0 = warp_find_row(wk.rows(*I), I->p, t0 - base_t);
     {  // the block of the tile's first row and its neighbours' live bits (whole warp)
       const int d0 = I->deg[i0];
       if (d0 <= kBlkD) {
@@ -1334,18 +1340,18 @@ __device__ __forceinline__ void tests_set(const Launch &L, unsigned long long *r
       }
     }
     const bool active = t < tend;
-    const bool same = t < L.work_prefix[b + 1];
-    int64_t i = lane_find_row(rw_c ? rw_c : I->row_work, I->p, i0, (active && same ? t : t0) - base_t, active && same);
+    const bool same = t < wk.end(b);
+    int64_t i = lane_find_row(wk.rows(*I), I->p, i0, (active && same ? t : t0) - base_t, active && same);
     if (active && !same) {  // the tile runs into the next instance
-      b = find_inst_u(L.work_prefix, L.count, t);
+      b = wk.inst(t);
       I = inst_of(L, b);
-      base_t = L.work_prefix[b];
-      i = find_row(rw_c ? rw_c : I->row_work, I->p, t - base_t);
+      base_t = wk.begin(b);
+      i = find_row(wk.rows(*I), I->p, t - base_t);
     }
     if (active) {
       int d = I->deg[i];
       int base = I->rowptr[i];
-      unrank_lex_fast(t - base_t - (rw_c ? rw_c : I->row_work)[i], l, d, pos);
+      unrank_lex_fast(t - base_t - wk.rows(*I)[i], l, d, pos);
       bool staged = i == blk_i && b == blk_b;
       uint64_t live = staged ? blk_live : row_live_mask(*I, i, base, d);
       int ci = 0;  // lowest member changed since the last unit (factor rows below are valid)
@@ -1453,13 +1459,13 @@ __device__ __forceinline__ void tests_set(const Launch &L, unsigned long long *r
         if (++t >= tend) break;
         ci = next_lex(l, d, pos);
         if (ci < 0) {  // the row's last set: the next row with tests, possibly of the next instance
-          if (t >= L.work_prefix[b + 1]) {
-            b = find_inst_u(L.work_prefix, L.count, t);
+          if (t >= wk.end(b)) {
+            b = wk.inst(t);
             I = inst_of(L, b);
-            base_t = L.work_prefix[b];
-            i = find_row(rw_c ? rw_c : I->row_work, I->p, t - base_t);
+            base_t = wk.begin(b);
+            i = find_row(wk.rows(*I), I->p, t - base_t);
           } else {
-            i = find_row_from(rw_c ? rw_c : I->row_work, I->p, i, t - base_t);
+            i = find_row_from(wk.rows(*I), I->p, i, t - base_t);
           }
           d = I->deg[i];
           base = I->rowptr[i];

@@ -296,7 +296,7 @@ struct Launch {
   long long rq_vcap;
   const long long *seg_prefix;      // scan segments  sum ceil(p / kSegRows) (count + 1)
   SegAgg *seg;                      // this level's segment sums (zeroed before the level)
-  int row_cache;                    // the CI tests keep the row offsets in shared memory
+  int row_cache;                    // the blocks form the row offsets themselves (own_scan)
   long long total_rows, total_segs; // row_prefix[count], seg_prefix[count]
   const TuneEntry *tune;            // the context's tile-policy table (kTunePB x kLevels x kTuneDB)
   TuneEntry force;                  // tile_cap > 0: this policy for the level, whatever the table says
@@ -331,7 +331,7 @@ __device__ __forceinline__ long long seg_begin(const Launch &L, int b) { return 
 __device__ __forceinline__ long long seg_end(const Launch &L, int b) {
   return L.count == 1 ? L.total_segs : L.seg_prefix[b + 1];
 }
-// row offsets a level kernel of levels >= 2 caches in shared memory (one instance)
+// row offsets of one instance that a level kernel's blocks (levels >= 2) form in their shared memory
 constexpr int kRowCache = 5120;
 
 __device__ __forceinline__ int find_inst(const long long *prefix, int count, long long t) {

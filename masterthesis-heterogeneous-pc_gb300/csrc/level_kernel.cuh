@@ -26,14 +26,25 @@ __global__ void __launch_bounds__(kThreads, variant_blocks(LT, V, kSetBlocks<LT>
   rebuild_phase(L, kUnits, LT == 1 && (V & kWide) != 0);
   if (!grid_barrier(L, epoch)) return;
   if (stamp) L.lc->t_rebuilt = globaltimer_ns();
-  scan_phase(L, kUnits);
-  if (!grid_barrier(L, epoch)) return;
+  // (level 1 leaves its shared memory to the L1 cache, the wide-row kernels need the queue of the scan)
+  constexpr bool kOwn = LT != 1 && (V == kSetOrder || !(V & kWide));
+  int max_deg = 0;
+  Work wk{0, nullptr, L.work_prefix, L.count};
+  if (kOwn && L.row_cache) {
+    wk.total = own_scan(L, kUnits, rw_smem, &max_deg);
+    wk.own = rw_smem;
+  } else {
+    scan_phase(L, kUnits);
+    if (!grid_barrier(L, epoch)) return;
+    wk.total = L.work_prefix[L.count];
+    max_deg = *(volatile const int *)&L.lc->max_deg;
+  }
   if (stamp) L.lc->t_scanned = globaltimer_ns();
-  const TuneEntry te = tile_policy(L);
+  const TuneEntry te = tile_policy(L, max_deg);
   if constexpr (V == kSetOrder) {
     static_assert(MIXED && LT >= 2 && LT <= kSetTop, "the set order runs levels 2-24 in mixed precision");
     __shared__ TestSmem<LT, true> sm;
-    tests_set<LT>(L, rw_smem, te, sm);
+    tests_set<LT>(L, wk, te, sm);
   } else if constexpr (LT == 1 && (V & kWide) != 0) {
     static_assert(MIXED, "the wide-row kernels run in mixed precision");
     tests_l1_wide<(V & kQueueOnly) != 0>(L, *reinterpret_cast<Wide1Smem *>(rw_smem));
@@ -42,12 +53,16 @@ __global__ void __launch_bounds__(kThreads, variant_blocks(LT, V, kSetBlocks<LT>
     static_assert(sizeof(Wide2Smem) <= sizeof(sm.blk), "the wide rows' scalars stand where the staged blocks do");
     tests_l2_wide(L, *reinterpret_cast<Wide2Smem *>(sm.blk), sm.pend[0], sm.np);
     __syncthreads();
-    tests_generic<2, true>(L, rw_smem, te, sm);
+    tests_generic<2, true>(L, wk, te, sm);
   } else if constexpr (LT == 1 && (V & 3) != kL1Chunked) {  // level 1 keeps the SM's on-chip memory for L1 cache
-    tests_l1<MIXED, (V & 3) == kL1Prefetch, (V & kQueueOnly) != 0>(L, nullptr, te);
+    tests_l1<MIXED, (V & 3) == kL1Prefetch, (V & kQueueOnly) != 0>(L, wk, te);
   } else {
     __shared__ TestSmem<LT, MIXED> sm;
-    tests_generic<LT, MIXED>(L, LT == 1 ? nullptr : rw_smem, te, sm);
+    tests_generic<LT, MIXED>(L, wk, te, sm);
+  }
+  if (kOwn && wk.own && blockIdx.x == gridDim.x - 1 && threadIdx.x < 32) {
+    __syncwarp();
+    own_summary(L, wk.total, max_deg);
   }
   __syncthreads();
   if (threadIdx.x == 0) atomicMax(&L.lc->t_end, globaltimer_ns());

@@ -14,6 +14,9 @@
 //            instance's level summary, and (one block) the prefix of the instances'
 //            unit counts.
 //
+// A single instance of up to kRowCache - 1 rows has no scan phase: every block forms the prefix
+// for itself (own_scan).
+//
 // Together they replace compactCUTiled (src/independence/compact.cu:4-89), which
 // rebuilds the reference's dense adj_compact rows with one thread block per row.
 #pragma once
@@ -400,6 +403,80 @@ __device__ __forceinline__ void scan_phase(const Launch &L, int units) {
       C.rec_begin = *(volatile unsigned long long *)&I.g->rec_count;
     }
     __syncthreads();
+  }
+}
+
+// The scan of a single instance of up to kRowCache - 1 rows by every block for itself, into its
+// shared memory (rw, p + 1 offsets): no second grid barrier, no copy of the offsets from global
+// memory: with p = 50 the scan and its barrier took 4.8 us of a level's 24, this takes 1.5; a skeleton
+// of p = 50, levels 0-6, 236 -> 217 us as a whole call. The loops stay rolled: a level of a few tests
+// spends much of its time on fetching instructions. Returns the number of units, the largest degree in *max_deg.
+__device__ __forceinline__ unsigned long long own_scan(const Launch &L, int units, unsigned long long *rw,
+                                                       int *max_deg) {
+  __shared__ int s_max[kLevelThreads / 32];
+  const Inst &I = *inst_of(L, 0);
+  const int tid = threadIdx.x, p = (int)I.p, level = L.level;
+  const bool csr = csr_overflow(I);
+  int md = 0, over = 0;
+#pragma unroll 4
+  for (int r = tid; r < p; r += kLevelThreads) {
+    const int d = __ldcg(I.deg + r);
+    md = max(md, d);
+    rw[r + 1] = (unsigned long long)d;
+  }
+  md = __reduce_max_sync(0xffffffffu, md);
+  if ((tid & 31) == 0) s_max[tid >> 5] = md;
+  __syncthreads();
+  // each thread a run of rows: their units, then their offsets
+  const int per = (p + kLevelThreads - 1) / kLevelThreads, lo = min(p, tid * per), hi = min(p, lo + per);
+  unsigned long long sum = 0;
+#pragma unroll 1
+  for (int r = lo; r < hi; ++r) {
+    const int d = (int)rw[r + 1];
+    unsigned long long w = row_tests(d, level, L.row_work_limit, &over);
+    if (units == kUnitSets && w) w = row_sets(d, level);
+    rw[r + 1] = w;
+    sum += w;
+  }
+  const bool bad = __syncthreads_or(over != 0) || csr;
+  unsigned long long total;
+  unsigned long long run = block_exclusive_scan(sum, &total);
+#pragma unroll 1
+  for (int r = lo; r < hi; ++r) {
+    run += rw[r + 1];
+    rw[r + 1] = bad ? 0ull : run;
+  }
+  if (tid == 0) rw[0] = 0;
+  md = 0;
+#pragma unroll
+  for (int q = 0; q < kLevelThreads / 32; ++q) md = max(md, s_max[q]);
+  *max_deg = md;
+  __syncthreads();
+  return bad ? 0ull : total;
+}
+
+// The level's summary beside own_scan, by one warp of the last block when its tests are done: it
+// is read by the next level and the host. (The counters of the CI tests are zero since the run's
+// start: other blocks count already.)
+__device__ __forceinline__ void own_summary(const Launch &L, unsigned long long total, int max_deg) {
+  const Inst &I = *inst_of(L, 0);
+  const int level = L.level;
+  const bool csr = csr_overflow(I);
+  const InstSums rs = warp_inst_sums(L, 0, 0, false);
+  if ((threadIdx.x & 31) == 0) {
+    DevCounters &C = I.ctr[level];
+    const bool bad = csr || rs.over;
+    // the lists just rebuilt are the instance's snapshot (unless they overflowed)
+    I.g->snap = bad ? 0ull : I.snap_epoch;
+    if (rs.over) atomicOr(&I.g->err, kErrWorkOverflow);
+    if (csr) atomicOr(&I.g->err, kErrCsrOverflow);
+    C.edges2 = rs.deg;
+    C.work_total = bad ? 0ull : rs.work;
+    C.max_deg = rs.max_deg;
+    C.rows = rs.rows;
+    L.work_prefix[0] = 0;
+    L.work_prefix[1] = total;
+    L.lc->max_deg = max_deg;
   }
 }
 
