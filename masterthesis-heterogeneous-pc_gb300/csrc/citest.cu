@@ -508,6 +508,23 @@ __global__ void __launch_bounds__(kRetestWarps * 32, 2) retest_kernel(const __gr
   }
 }
 
+// Level-1 re-tests of instances with an FP64 matrix (mixed precision from a matrix or with the
+// FP64-accurate Gram): a thread an item, the three entries read from the matrix, decided as
+// tests_l1 decides them inline.
+__global__ void __launch_bounds__(128) retest_matrix_kernel(const __grid_constant__ Launch L) {
+  unsigned long long count = L.lc->rq_count;
+  if (count > (unsigned long long)L.rq_cap) count = (unsigned long long)L.rq_cap;
+  for (unsigned long long q = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; q < count;
+       q += (unsigned long long)gridDim.x * blockDim.x) {
+    const RetestItem *it = L.rq + q;
+    const Inst &I = *inst_of(L, it->inst);
+    double pv;
+    if (live_bit(I.adj, I.W, it->i, it->j) && exact_remove_fast<1>(I, it->i, it->j, it->ids, 1, &pv) &&
+        claim_edge<false>(I, it->i, it->j))
+      write_record(I, 1, it->i, it->j, it->ids, 1, pv);
+  }
+}
+
 template <bool MIXED>
 void *kernel_for(int level, int l1_variant) {
   if (MIXED && l1_variant == kSetOrder && level >= 2 && level <= kSetTop) {
@@ -607,6 +624,12 @@ hpc_status launch_retest(const Launch &L, int sms, cudaStream_t s) {
   else
     retest_kernel<HPC_MAX_LEVEL><<<sms * 4, kRetestWarps * 32, smem, s>>>(L);
   HPC_LAUNCH_CHECK("retest_kernel");
+  return HPC_OK;
+}
+
+hpc_status launch_retest_matrix(const Launch &L, int sms, cudaStream_t s) {
+  retest_matrix_kernel<<<sms * 2, 128, 0, s>>>(L);
+  HPC_LAUNCH_CHECK("retest_matrix_kernel");
   return HPC_OK;
 }
 

@@ -339,7 +339,7 @@ hpc_status enqueue_level(hpc_ctx *c, int level, bool timed) {
   // level 1: the queue-only build of the interleaved variants where the re-tests are
   // queued and a queue overflow can be rerun
   const bool wide = (level == 1 && c->wide1) || (level == 2 && c->wide2 && !set);
-  const bool qo = level == 1 && (wide || c->l1v_now != kL1Chunked) && effective_set_from(c) > 0;
+  const bool qo = level == 1 && (wide || c->l1v_now != kL1Chunked) && (effective_set_from(c) > 0 || c->defer1);
   const int l1v = wide ? kWide : c->l1v_now;
   const int var = level == 1 ? (qo ? l1v | kQueueOnly : l1v) : set ? kSetOrder : wide ? kWide : kL1Interleaved;
   const int grid = wide         ? c->citest_grid_wide[level == 2 ? 2 : qo ? 1 : 0]
@@ -349,8 +349,10 @@ hpc_status enqueue_level(hpc_ctx *c, int level, bool timed) {
   if ((s = launch_level(L, c->opts.precision, grid, var, c->stream)) != HPC_OK) return s;
   if (timed) HPC_CUDA(cudaEventRecord(ev[3], c->stream));
   if (queue && (s = launch_retest(L, c->sm_count, c->stream)) != HPC_OK) return s;
+  const bool matrix = qo && c->cor64_valid;
+  if (matrix && (s = launch_retest_matrix(L, c->sm_count, c->stream)) != HPC_OK) return s;
   if (timed) HPC_CUDA(cudaEventRecord(ev[2], c->stream));
-  c->timings.launches += queue ? 2 : 1;
+  c->timings.launches += queue || matrix ? 2 : 1;
   return HPC_OK;
 }
 
@@ -596,6 +598,34 @@ hpc_status choose_wide(hpc_ctx *c) {
   return HPC_OK;
 }
 
+// Whether level 1 of a context with an FP64 matrix (mixed precision) queues its undecided tests for
+// a kernel of their own instead of re-testing inline: the inline FP64 re-test costs the
+// interleaved kernel registers (it spills) and a warp stops for its one lane. It takes a launch
+// more, so from kDefer1Tests potential tests (about edges2^2 / p) on; measured (p = 2000, 1.3e7 of them:
+// 129 us inline, 92 + 10 us with the kernel after it). A queue that overflows is rerun inline (set_off), as in tensor-core mode.
+constexpr double kDefer1Tests = 4e6;
+void choose_defer1(hpc_ctx *c) {
+  c->defer1 = false;
+  if (c->opts.precision != HPC_PREC_MIXED || !c->cor64_valid || c->set_off || c->level_by_level || !c->level0_known ||
+      set_order_from() == 0)
+    return;
+  double tests = 0.0;
+  long long p2 = 0;
+  for (int b = 0; b < c->count; ++b) {
+    const double e2 = (double)c->ctr_host[(size_t)b * kLevels].edges2;
+    tests += e2 * e2 / (double)c->ih[b].p;
+    p2 += c->ih[b].p * c->ih[b].p;
+  }
+  if (tests < kDefer1Tests) return;
+  if (!c->rq) {
+    const long long cap = std::min<long long>(1ll << 20, std::max<long long>(1ll << 14, p2 / 16));
+    if (dev_alloc(&c->rq, cap, "re-test queue") != HPC_OK) return;  // re-tests inline, then
+    c->rq_cap = cap;
+    ++c->inst_version;  // a captured graph holds the queue pointer
+  }
+  c->defer1 = true;
+}
+
 // Run levels first..last with one host sync at the end; the whole sequence 0..last
 // is captured once into a CUDA graph and replayed while the buffers stay in place.
 // `finalize` appends the FP64 p-values of the FP32-decided removals (and their FP64
@@ -607,6 +637,7 @@ hpc_status run_levels(hpc_ctx *c, int first, int last, bool use_graph, bool wait
   if ((s = sync_tune(c)) != HPC_OK) return s;
   c->l1v_now = level1_variant(c);
   if (last >= 1 && (s = choose_wide(c)) != HPC_OK) return s;
+  if (last >= 1) choose_defer1(c);
   finalize = finalize && last >= 1 && c->recs;
   auto enqueue_all = [&](bool timed) -> hpc_status {
     if (first == 0) {  // a skeleton from the start: its counters and records begin at zero
@@ -628,7 +659,7 @@ hpc_status run_levels(hpc_ctx *c, int first, int last, bool use_graph, bool wait
   if (use_graph && c->graphs_enabled && first == 0 && capturable(c->stream)) {
     const bool valid = c->graph && c->graph_top == last && c->graph_stream == c->stream &&
                        c->graph_version == c->inst_version && c->graph_l1v == (c->wide1 ? kWide : c->l1v_now) &&
-                       c->graph_wide2 == c->wide2 &&
+                       c->graph_wide2 == c->wide2 && c->graph_defer1 == c->defer1 &&
                        c->graph_set_mask == set_mask(c, last) &&
                        c->graph_final == finalize;
     if (!valid) {
@@ -656,6 +687,7 @@ hpc_status run_levels(hpc_ctx *c, int first, int last, bool use_graph, bool wait
       c->graph_version = c->inst_version;
       c->graph_l1v = c->wide1 ? kWide : c->l1v_now;
       c->graph_wide2 = c->wide2;
+      c->graph_defer1 = c->defer1;
       c->graph_set_mask = set_mask(c, last);
       c->graph_final = finalize;
     }

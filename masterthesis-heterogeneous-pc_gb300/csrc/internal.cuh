@@ -412,6 +412,7 @@ hpc_status launch_expand_adjacency(const uint32_t *adj, int64_t p, int W, uint8_
 // l1_variant: level 1's kernel (kL1Interleaved, kL1Prefetch or kL1Chunked, from the tile policy).
 hpc_status launch_level(const Launch &L, int precision, int grid, int l1_variant, cudaStream_t s);
 hpc_status launch_retest(const Launch &L, int sms, cudaStream_t s);
+hpc_status launch_retest_matrix(const Launch &L, int sms, cudaStream_t s);  // level 1, from FP64 matrices
 void retest_setup();  // once per context creation, before any launch_retest
 hpc_status launch_finalize_records(const Inst *inst, int count, cudaStream_t s);
 // every instance's records packed back to back: instance b's first record goes to
@@ -566,6 +567,7 @@ struct hpc_ctx {
   int citest_grid_l1[3] = {};     // grids of the level-1 kernel variants (kL1*)
   int citest_grid_l1q[2] = {};    // ... and of the queue-only ones (kL1Interleaved, kL1Prefetch | kQueueOnly)
   int citest_grid_wide[3] = {};   // ... of the wide-row kernels (level 1, 1 queue-only at index 0, level 2)
+  bool defer1 = false;            // level 1 of the runs being queued: re-tests queued beside an FP64 matrix
   bool wide1 = false, wide2 = false;  // level 1 / level 2 of the runs being queued: the wide-row kernels
   bool level0_known = false;      // ctr_host holds a level-0 result
   int wide_cols = 0;              // columns of an item of level 1's
@@ -579,6 +581,7 @@ struct hpc_ctx {
   int l1v_now = 0;                // the level-1 kernel variant of the runs being queued
   int graph_l1v = 0;              // ... and of the captured graph
   bool graph_wide2 = false;       // ... whose level 2 runs the wide-row kernel
+  bool graph_defer1 = false;      // ... whose level 1 queues its re-tests beside an FP64 matrix
   unsigned int graph_set_mask = 0;  // the set-order levels of the captured graph (bit l)
   int deg_seen[HPC_MAX_LEVEL + 1];  // largest degree at each level's start in the last run (-1: unknown)
   bool set_off = false;           // the set order turned off (a re-test queue overflow)

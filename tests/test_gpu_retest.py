@@ -27,3 +27,26 @@ def test_oracle(p, n, factors, margin):
         assert np.array_equal(sk.adjacency(), want.adj)
     assert orc.verify_sepsets(Cm, n, 0.05, sk.sepset_records()).all()
     sk.close()
+
+
+@pytest.mark.parametrize("entries", [None, 16])
+@pytest.mark.parametrize("p,margin", [(260, 1e-3), (321, 0.05)])
+def test_level_1_deferred_beside_a_matrix(p, margin, entries):
+    """Mixed precision with an FP64 matrix and millions of level-1 tests: the re-tests go through the
+    queue, and inline where it is too small."""
+    n = 400
+    rng = np.random.default_rng(p)
+    X = rng.uniform(0.2, 0.9, (p, 1)) * rng.standard_normal((1, n)) + rng.standard_normal((p, n))
+    Cm = orc.correlation(X)
+    want = orc.run(Cm, n, 0.05, 1)
+    sk = hg.SkeletonCalculator(p, n, alpha=0.05, max_level=1, retest_margin=margin)
+    sk.add_correlation_matrix(Cm)
+    sk.run()
+    if entries:
+        assert hg.lib().hpc_debug_set_retest_queue(sk.handle, entries) == 0
+    for _ in range(3):  # eager (or overflowing), captured, replayed
+        sk.reset()
+        sk.run()
+        assert np.array_equal(sk.adjacency(), want.adj)
+    assert orc.verify_sepsets(Cm, n, 0.05, sk.sepset_records()).all()
+    sk.close()
