@@ -855,7 +855,8 @@ __device__ __forceinline__ void tests_generic(const Launch &L, const Work &wk, c
             pv = -1.0 - (double)rr;
           } else if (res == 2) {
             if (MIXED) ++retests;
-            if (!(MIXED && !I->cor64 && push_retest(L, b, i, j, ids, l))) rm = exact_remove_fast<LA>(*I, i, j, ids, l, &pv);
+            if (!(MIXED && !I->cor64 && push_retest(L, b, i, j, ids, l)))
+              rm = exact_remove_fast<LA>(*I, i, j, ids, l, &pv);
           }
           if (rm) {
             if (claim_edge<LT != 1>(*I, i, j)) {
@@ -1131,8 +1132,8 @@ __device__ __forceinline__ void tests_l1(const Launch &L, const Work &wk, const 
 
 // ---------------------------------------------------------------------------
 // The set order of a level's CI tests (levels 2-24, mixed precision; the kSetOrder
-// kernels, launched from the level set_order_from() on). The flattened index runs over (instance, row i, l-subset S of the row's snapshot neighbours in
-// lexicographic order), and one unit runs the tests (i, j | S) for every live
+// kernels, launched from the level set_order_from() on). The flattened index runs over
+// (instance, row i, l-subset S of the row's snapshot neighbours in lexicographic order), and one unit runs the tests (i, j | S) for every live
 // neighbour j outside S, in ascending order. A row of degree d > l has C(d, l) units
 // holding C(d, l) (d - l) = d C(d - 1, l) tests: every test of the edge order once,
 // each in the same FP32 arithmetic -- the Cholesky factor of S and w_i formed as

@@ -553,9 +553,9 @@ hpc_status sync_tune(hpc_ctx *c) {
 // run), level 2 by its degrees in the last run -- before a first run, where level 1 is wide.
 // Level 2 needs kWide2Rows rows of a mean degree of kWide2Deg to keep its blocks busy (measured,
 // ordinary against wide: mean degree 41 of 1000 rows 405 / 455 us, 35 of 700 248 / 508 us; 65 of 1500
-// 1794 / 966 us, 85 of 2000 4.9 / 2.3 ms, 51 of 2000 1.92 / 1.95 ms, 42 of 8000 7.0 / 2.1 ms). (The kernel of level 2 takes the wide rows and leaves the others to the
-// ordinary body, so a wrong guess costs time only.) Without room for the buffers the ordinary
-// kernels run.
+// 1794 / 966 us, 85 of 2000 4.9 / 2.3 ms, 51 of 2000 1.92 / 1.95 ms, 42 of 8000 7.0 / 2.1 ms). (The
+// kernel of level 2 takes the wide rows and leaves the others to the ordinary body, so a wrong guess
+// costs time only.) Without room for the buffers the ordinary kernels run.
 constexpr long long kWide2Rows = 1500;
 constexpr double kWide2Deg = 40.0;
 hpc_status choose_wide(hpc_ctx *c) {
@@ -601,8 +601,9 @@ hpc_status choose_wide(hpc_ctx *c) {
 // Whether level 1 of a context with an FP64 matrix (mixed precision) queues its undecided tests for
 // a kernel of their own instead of re-testing inline: the inline FP64 re-test costs the
 // interleaved kernel registers (it spills) and a warp stops for its one lane. It takes a launch
-// more, so from kDefer1Tests potential tests (about edges2^2 / p) on; measured (p = 2000, 1.3e7 of them:
-// 129 us inline, 92 + 10 us with the kernel after it). A queue that overflows is rerun inline (set_off), as in tensor-core mode.
+// more, so from kDefer1Tests potential tests (about edges2^2 / p) on; measured (p = 2000, 1.3e7 of
+// them): 129 us inline, 92 + 10 us with the kernel after it. A queue that overflows is rerun inline
+// (set_off), as in tensor-core mode.
 constexpr double kDefer1Tests = 4e6;
 void choose_defer1(hpc_ctx *c) {
   c->defer1 = false;

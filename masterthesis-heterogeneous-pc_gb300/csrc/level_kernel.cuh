@@ -17,7 +17,7 @@ constexpr int variant_blocks(int lt, int v, int set_blocks) {  // resident block
 template <int LT, bool MIXED, int V = kL1Interleaved>
 __global__ void __launch_bounds__(kThreads, variant_blocks(LT, V, kSetBlocks<LT>))
     level_kernel(const __grid_constant__ Launch L) {
-  // kRowCache row offsets, or the wide level-1 body's chunk
+  // the row offsets of own_scan, or the wide bodies' chunk and ring
   extern __shared__ __align__(16) unsigned long long rw_smem[];
   constexpr int kUnits = V == kSetOrder ? kUnitSets : (LT == 2 && V == kWide) ? kUnitNarrow : kUnitTests;
   unsigned int epoch = 0;
