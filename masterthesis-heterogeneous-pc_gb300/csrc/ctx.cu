@@ -264,6 +264,12 @@ unsigned int set_mask(const hpc_ctx *c, int last) {
   return m;
 }
 
+// Level 1 of the runs being queued: the queue-only build of its kernel, where the re-tests are queued
+// and a queue overflow can be rerun.
+bool queue_only1(const hpc_ctx *c) {
+  return (c->wide1 || c->l1v_now != kL1Chunked) && (effective_set_from(c) > 0 || c->defer1);
+}
+
 Launch make_launch(hpc_ctx *c, int level) {
   Launch L{};
   L.inst = c->inst;
@@ -336,10 +342,8 @@ hpc_status enqueue_level(hpc_ctx *c, int level, bool timed) {
   // snapshot rebuild, test-count scan and CI tests in one launch
   if (timed) HPC_CUDA(cudaEventRecord(ev[1], c->stream));
   const bool set = set_at(c, level);
-  // level 1: the queue-only build of the interleaved variants where the re-tests are
-  // queued and a queue overflow can be rerun
   const bool wide = (level == 1 && c->wide1) || (level == 2 && c->wide2 && !set);
-  const bool qo = level == 1 && (wide || c->l1v_now != kL1Chunked) && (effective_set_from(c) > 0 || c->defer1);
+  const bool qo = level == 1 && queue_only1(c);
   const int l1v = wide ? kWide : c->l1v_now;
   const int var = level == 1 ? (qo ? l1v | kQueueOnly : l1v) : set ? kSetOrder : wide ? kWide : kL1Interleaved;
   const int grid = wide         ? c->citest_grid_wide[level == 2 ? 2 : qo ? 1 : 0]
@@ -660,7 +664,7 @@ hpc_status run_levels(hpc_ctx *c, int first, int last, bool use_graph, bool wait
   if (use_graph && c->graphs_enabled && first == 0 && capturable(c->stream)) {
     const bool valid = c->graph && c->graph_top == last && c->graph_stream == c->stream &&
                        c->graph_version == c->inst_version && c->graph_l1v == (c->wide1 ? kWide : c->l1v_now) &&
-                       c->graph_wide2 == c->wide2 && c->graph_defer1 == c->defer1 &&
+                       c->graph_wide2 == c->wide2 && c->graph_qo1 == queue_only1(c) &&
                        c->graph_set_mask == set_mask(c, last) &&
                        c->graph_final == finalize;
     if (!valid) {
@@ -688,7 +692,7 @@ hpc_status run_levels(hpc_ctx *c, int first, int last, bool use_graph, bool wait
       c->graph_version = c->inst_version;
       c->graph_l1v = c->wide1 ? kWide : c->l1v_now;
       c->graph_wide2 = c->wide2;
-      c->graph_defer1 = c->defer1;
+      c->graph_qo1 = queue_only1(c);
       c->graph_set_mask = set_mask(c, last);
       c->graph_final = finalize;
     }

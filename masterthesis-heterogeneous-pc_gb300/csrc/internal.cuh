@@ -581,7 +581,7 @@ struct hpc_ctx {
   int l1v_now = 0;                // the level-1 kernel variant of the runs being queued
   int graph_l1v = 0;              // ... and of the captured graph
   bool graph_wide2 = false;       // ... whose level 2 runs the wide-row kernel
-  bool graph_defer1 = false;      // ... whose level 1 queues its re-tests beside an FP64 matrix
+  bool graph_qo1 = false;         // ... whose level 1 runs the queue-only build
   unsigned int graph_set_mask = 0;  // the set-order levels of the captured graph (bit l)
   int deg_seen[HPC_MAX_LEVEL + 1];  // largest degree at each level's start in the last run (-1: unknown)
   bool set_off = false;           // the set order turned off (a re-test queue overflow)
