@@ -231,12 +231,14 @@ hpc_status hpc_tune_clear(void);
  * the same key. */
 hpc_status hpc_tune_save(const char *path);
 hpc_status hpc_tune_load(const char *path);
-/* Forces one policy on every level of the context's runs (NULL = the table again). */
+/* Forces one policy on every level of the context's runs (NULL = the table again). Levels 1 and 2
+ * then run the kernels that read a policy, on wide rows too (whose own kernels read none). */
 hpc_status hpc_ctx_set_tune(hpc_ctx *ctx, const hpc_tune_params *force);
 /* Autotuner: runs the context's skeleton (on its current correlation, kernel by
  * kernel) once per candidate policy in each of `reps` rounds, times every level's
  * CI-test kernel with CUDA events, and stores for each level the candidate with the
- * smallest median time under the level's key. cands/ncands: the candidates (NULL = the built-in grid: tile_cap
+ * smallest median time under the level's key. The candidates run as forced policies (above), so a
+ * stored policy was timed on a kernel that reads it. cands/ncands: the candidates (NULL = the built-in grid: tile_cap
  * 16, 64, 256, 1024 x tiles_per_lane 2, 4, 8 x level-1 kernel interleaved,
  * interleaved with prefetch, chunked). chosen (optional,
  * HPC_MAX_LEVEL + 1 entries) receives each level's choice (zeros for levels not run);

@@ -565,7 +565,9 @@ constexpr double kWide2Deg = 40.0;
 hpc_status choose_wide(hpc_ctx *c) {
   c->wide1 = c->wide2 = false;
   if (c->opts.precision == HPC_PREC_FP64) return HPC_OK;
-  const bool forced_policy = c->tune_force.tile_cap > 0 && !c->tuning;  // a forced policy picks its kernels
+  // a forced policy picks its kernels, those that read it: hpc_autotune's candidates among them, whose
+  // times are stored for every context and server launch of the same sizes
+  const bool forced_policy = c->tune_force.tile_cap > 0;
   std::vector<WideShape> sh((size_t)c->count);
   for (int b = 0; b < c->count; ++b)
     sh[b] = WideShape{c->ih[b].p, c->level0_known ? (int64_t)c->ctr_host[(size_t)b * kLevels].edges2 : 0};
@@ -1250,7 +1252,6 @@ hpc_status hpc_autotune(hpc_ctx *c, const hpc_tune_params *cands, int ncands, in
   }
   const bool graphs = c->graphs_enabled;
   const TuneEntry force0 = c->tune_force;
-  c->tuning = true;
   c->graphs_enabled = false;  // kernel by kernel: every level's kernels are timed
   // every candidate's level times, the candidates taken in turn within each round (so
   // that a drift over the tuning run touches them alike); per level the candidate with
@@ -1291,7 +1292,6 @@ hpc_status hpc_autotune(hpc_ctx *c, const hpc_tune_params *cands, int ncands, in
     }
   }
   c->tune_force = force0;
-  c->tuning = false;
   c->graphs_enabled = graphs;
   ++c->inst_version;
   const hpc_status reset = hpc_ctx_reset(c);

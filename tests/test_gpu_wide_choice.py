@@ -1,0 +1,50 @@
+"""Which kernels levels 1 and 2 run, read from the tests that a level executes: on a complete graph
+that loses no edge at level 1 the ordinary kernels run every test from both of its rows, the
+kernel for wide rows once."""
+import ctypes as C
+import re
+
+import numpy as np
+import pytest
+
+import heterogpc as hg
+
+pytestmark = pytest.mark.gpu
+
+# equicorrelation 1/2: 1/3 given one variable, 1/4 given two; the critical value lies between them,
+# so level 1 keeps every edge and every test of level 2 removes its edge
+N_OBS, ALPHA = 100, 0.0033
+
+
+def _equicorrelation(p):
+    return 0.5 * np.ones((p, p)) + 0.5 * np.eye(p)
+
+
+def _context(p, max_level, verbose=False):
+    sk = hg.SkeletonCalculator(p, N_OBS, alpha=ALPHA, max_level=max_level, verbose=verbose)
+    sk.add_correlation_matrix(_equicorrelation(p))
+    return sk
+
+
+def _level1(sk):
+    """executed / potential tests of level 1 in one more run"""
+    sk.reset()
+    st = sk.run()[1]
+    assert st["edges_after"] == st["edges_before"] == sk.p * (sk.p - 1) // 2
+    return st["executed_tests"] / st["potential_tests"]
+
+
+def test_autotune_times_the_kernels_that_read_the_policies(capfd):
+    hg.tune_clear()
+    sk = _context(1200, 1, verbose=True)
+    assert _level1(sk) == 0.5  # wide rows by the rule
+    C.CDLL(None).fflush(None)
+    capfd.readouterr()
+    sk.autotune([{"tile_cap": 16, "tiles_per_lane": 4, "edge_lanes": 32, "l1_prefetch": 0},
+                 {"tile_cap": 64, "tiles_per_lane": 8, "edge_lanes": 32, "l1_prefetch": 1}], reps=2)
+    C.CDLL(None).fflush(None)
+    runs = re.findall(r"level 1: .* tests (\d+) of (\d+)", capfd.readouterr().out)
+    assert len(runs) == 4 and all(done == potential for done, potential in runs)
+    assert _level1(sk) == 0.5  # and wide again after it
+    sk.close()
+    hg.tune_clear()
