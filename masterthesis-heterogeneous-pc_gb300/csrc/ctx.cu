@@ -559,7 +559,8 @@ hpc_status sync_tune(hpc_ctx *c) {
 // ordinary against wide: mean degree 41 of 1000 rows 405 / 455 us, 35 of 700 248 / 508 us; 65 of 1500
 // 1794 / 966 us, 85 of 2000 4.9 / 2.3 ms, 51 of 2000 1.92 / 1.95 ms, 42 of 8000 7.0 / 2.1 ms). (The
 // kernel of level 2 takes the wide rows and leaves the others to the ordinary body, so a wrong guess
-// costs time only.) Without room for the buffers the ordinary kernels run.
+// costs time only.) A level without room for its buffers runs the ordinary kernel, for the rest of the
+// context's life; the other level does not depend on it.
 constexpr long long kWide2Rows = 1500;
 constexpr double kWide2Deg = 40.0;
 hpc_status choose_wide(hpc_ctx *c) {
@@ -571,9 +572,11 @@ hpc_status choose_wide(hpc_ctx *c) {
   std::vector<WideShape> sh((size_t)c->count);
   for (int b = 0; b < c->count; ++b)
     sh[b] = WideShape{c->ih[b].p, c->level0_known ? (int64_t)c->ctr_host[(size_t)b * kLevels].edges2 : 0};
-  if (c->level0_known && !forced_policy && !c->wide_denied) {
-    c->wide1 = wide1_pays(sh.data(), c->count);
-    c->wide2 = c->deg_seen[2] >= 0 ? c->total_rows >= kWide2Rows && c->mean_deg2 >= kWide2Deg : c->wide1;
+  if (c->level0_known && !forced_policy) {
+    const bool pays1 = wide1_pays(sh.data(), c->count);
+    c->wide1 = pays1 && !c->wide1_denied;
+    c->wide2 = (c->deg_seen[2] >= 0 ? c->total_rows >= kWide2Rows && c->mean_deg2 >= kWide2Deg : pays1) &&
+               !c->wide2_denied;
   }
   if (c->wide_force1 >= 0) c->wide1 = c->wide_force1 > 0;
   if (c->wide_force2 >= 0) c->wide2 = c->wide_force2 > 0;
@@ -583,23 +586,27 @@ hpc_status choose_wide(hpc_ctx *c) {
     if (cols != c->wide_cols) ++c->inst_version;  // a launch parameter
     c->wide_cols = cols;
     if (!c->adj0) {
-      s = dev_alloc(&c->adj0, c->total_words, "adjacency snapshot");
-      if (s == HPC_OK && (s = write_inst_table(c)) != HPC_OK) return s;
+      if (dev_alloc(&c->adj0, c->total_words, "adjacency snapshot") != HPC_OK) {
+        c->wide1 = false;
+        c->wide1_denied = true;
+      } else if ((s = write_inst_table(c)) != HPC_OK) {
+        return s;
+      }
     }
   }
-  if (c->wide2 && !c->wide_scratch && s == HPC_OK) {
+  if (c->wide2 && !c->wide_scratch) {
     long long cap = 0;
     for (const auto &h : c->ih) cap += h.p * wide2_slices(h.p - 1, h.p);
-    if (!c->wide_items) s = dev_alloc(&c->wide_items, cap, "wide-row queue");
     c->wide_cap = cap;
     c->wide_floats = wide2_floats(c->p_max - 1);
-    if (s == HPC_OK) s = dev_alloc(&c->wide_scratch, c->wide_floats * c->citest_grid_wide[2], "wide-row scratch");
-    if (s == HPC_OK) ++c->inst_version;  // a captured graph holds no pointers to them
-  }
-  if (s != HPC_OK) {
-    c->wide1 = c->wide1 && c->adj0;
-    c->wide2 = c->wide2 && c->wide_scratch;
-    c->wide_denied = true;
+    if (dev_alloc(&c->wide_items, cap, "wide-row queue") != HPC_OK ||
+        dev_alloc(&c->wide_scratch, c->wide_floats * c->citest_grid_wide[2], "wide-row scratch") != HPC_OK) {
+      dev_free(c->wide_items);
+      c->wide2 = false;
+      c->wide2_denied = true;
+    } else {
+      ++c->inst_version;  // a captured graph holds no pointers to them
+    }
   }
   return HPC_OK;
 }

@@ -573,7 +573,7 @@ struct hpc_ctx {
   int wide_cols = 0;              // columns of an item of level 1's
   int wide_force1 = -1, wide_force2 = -1;  // test hook: 0 / 1 instead of the rules
   double mean_deg2 = 0.0;         // mean degree at level 2's start in the last run
-  bool wide_denied = false;       // no room for the wide-row kernels' buffers
+  bool wide1_denied = false, wide2_denied = false;  // no room for the wide-row kernels' buffers
   int64_t p_max = 0;
   int citest_grid_set[HPC_MAX_LEVEL + 1] = {};  // grids of the set-order kernels (levels 2-16)
   int l1_max_deg = -1;            // level-1 max degree of the last run (keys level 1's kernel choice)

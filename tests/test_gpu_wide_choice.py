@@ -34,6 +34,10 @@ def _level1(sk):
     return st["executed_tests"] / st["potential_tests"]
 
 
+def _set_wide(sk, l1, l2):
+    assert hg.lib().hpc_debug_set_wide(sk.handle, l1, l2) == 0
+
+
 def test_autotune_times_the_kernels_that_read_the_policies(capfd):
     hg.tune_clear()
     sk = _context(1200, 1, verbose=True)
@@ -48,3 +52,23 @@ def test_autotune_times_the_kernels_that_read_the_policies(capfd):
     assert _level1(sk) == 0.5  # and wide again after it
     sk.close()
     hg.tune_clear()
+
+
+def test_no_room_for_level_2_leaves_level_1_alone():
+    L = hg.lib()
+    sk = _context(1600, 2)
+    _set_wide(sk, 0, 0)
+    assert _level1(sk) == 1.0
+    _set_wide(sk, -1, -1)
+    live = L.hpc_debug_live_allocations()
+    L.hpc_debug_fail_allocation(3)  # after level 1's snapshot and level 2's queue: level 2's scratch
+    try:
+        assert _level1(sk) == 0.5
+    finally:
+        L.hpc_debug_fail_allocation(0)
+    assert sk.edge_count() == 0  # level 2 on the ordinary kernel
+    assert L.hpc_debug_live_allocations() == live + 1  # the snapshot; the queue went back
+    for _ in range(2):
+        assert _level1(sk) == 0.5 and sk.edge_count() == 0
+    assert L.hpc_debug_live_allocations() == live + 1
+    sk.close()
