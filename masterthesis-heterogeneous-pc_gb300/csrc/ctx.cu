@@ -563,7 +563,7 @@ hpc_status sync_tune(hpc_ctx *c) {
 // context's life; the other level does not depend on it.
 constexpr long long kWide2Rows = 1500;
 constexpr double kWide2Deg = 40.0;
-hpc_status choose_wide(hpc_ctx *c) {
+hpc_status choose_wide(hpc_ctx *c, int last) {
   c->wide1 = c->wide2 = false;
   if (c->opts.precision == HPC_PREC_FP64) return HPC_OK;
   // a forced policy picks its kernels, those that read it: hpc_autotune's candidates among them, whose
@@ -580,6 +580,7 @@ hpc_status choose_wide(hpc_ctx *c) {
   }
   if (c->wide_force1 >= 0) c->wide1 = c->wide_force1 > 0;
   if (c->wide_force2 >= 0) c->wide2 = c->wide_force2 > 0;
+  c->wide2 = c->wide2 && last >= 2;
   hpc_status s = HPC_OK;
   if (c->wide1) {
     const int cols = wide1_cols(sh.data(), c->count);
@@ -650,7 +651,7 @@ hpc_status run_levels(hpc_ctx *c, int first, int last, bool use_graph, bool wait
   hpc_status s;
   if ((s = sync_tune(c)) != HPC_OK) return s;
   c->l1v_now = level1_variant(c);
-  if (last >= 1 && (s = choose_wide(c)) != HPC_OK) return s;
+  if (last >= 1 && (s = choose_wide(c, last)) != HPC_OK) return s;
   if (last >= 1) choose_defer1(c);
   finalize = finalize && last >= 1 && c->recs;
   auto enqueue_all = [&](bool timed) -> hpc_status {

@@ -72,3 +72,16 @@ def test_no_room_for_level_2_leaves_level_1_alone():
         assert _level1(sk) == 0.5 and sk.edge_count() == 0
     assert L.hpc_debug_live_allocations() == live + 1
     sk.close()
+
+
+def test_no_level_2_buffers_below_level_2():
+    L = hg.lib()
+    live = []
+    for p in (1000, 1600):  # too few items for wide rows by the rule; enough
+        base = L.hpc_debug_live_allocations()
+        sk = _context(p, 1)
+        sk.run()
+        assert _level1(sk) == (1.0 if p == 1000 else 0.5)
+        live.append(L.hpc_debug_live_allocations() - base)
+        sk.close()
+    assert live[1] == live[0] + 1  # level 1's snapshot
