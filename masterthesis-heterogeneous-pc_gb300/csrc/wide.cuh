@@ -396,13 +396,15 @@ static_assert(kW2Slice % kThreads == 0 && kW2Slice / kThreads <= 32, "a thread w
 constexpr int kW2Ahead = 4;     // rows j in flight to a warp's ring
 struct Wide2Smem {
   float4 ring[kThreads / 32][kW2Ahead][32];  // rows j of the chunk, a lane's four b's each
-  float4 s[kThreads / 32][32][kW2A];         // per j of the warp's 32 and a: R_j, U'_j, -(1 - R_j^2), unused
+  // per j of the warp's 32 and a: R_j, U'_j, -(1 - R_j^2) and, for the first a, the j's tests in the chunk
+  float4 s[kThreads / 32][32][kW2A];
 };
 struct Wide2Lists {
   unsigned alive[kW2Slice / 32];  // the listed j's still live in this step
   uint16_t list[kW2Slice];        // the slice members alive at the step's start
   int total;
   unsigned item;
+  unsigned long long executed;    // the item's tests
 };
 
 // The tests of edge (i, j), j = neighbour xj - 1 of the row, with first members xa0 .. xa0 +
@@ -490,7 +492,10 @@ __device__ __forceinline__ void tests_l2_wide(const Launch &L, Wide2Smem &sm, Pe
   float *scratch = L.wide_scratch + (int64_t)blockIdx.x * L.wide_floats;
   for (;;) {
     __syncthreads();
-    if (tid == 0) ls.item = atomicAdd(&L.lc->wide_next, 1u);
+    if (tid == 0) {
+      ls.item = atomicAdd(&L.lc->wide_next, 1u);
+      ls.executed = 0;
+    }
     __syncthreads();
     const unsigned item = ls.item;
     if (item >= n_front + n_back) break;
@@ -507,7 +512,6 @@ __device__ __forceinline__ void tests_l2_wide(const Launch &L, Wide2Smem &sm, Pe
     wide2_copy(I, i, base, d, ld, 0, 1, 1, ri);
     wide2_copy(I, i, base, d, ld, 1 + it.slice, ns, m, rows);
     const float thr2 = quick_thr2(I, 2);
-    unsigned long long executed = 0;
     unsigned retests = 0;
     unsigned gone = 0;  // bit w: slice member tid + kThreads w is known to be removed
     for (int xs0 = 1; xs0 < d; xs0 += kW2Super) {
@@ -545,6 +549,7 @@ __device__ __forceinline__ void tests_l2_wide(const Launch &L, Wide2Smem &sm, Pe
         ria[a] = xa0 + a < d ? ri[xa0 + a] : 0.f;
         inv_i[a] = rsqrtf(fmaxf(1.0f - ria[a] * ria[a], 1e-6f));
       }
+      unsigned executed = 0;  // the lane's j's tests with the step's members a
       for (int x0 = (xa0 + 1) / kW2Chunk * kW2Chunk; x0 <= d; x0 += kW2Chunk) {
         const int xb = x0 + lane * 4;
         const bool load = xb < (int)ld;
@@ -609,7 +614,7 @@ __device__ __forceinline__ void tests_l2_wide(const Launch &L, Wide2Smem &sm, Pe
 #pragma unroll
           for (int k = 0; k < kW2Ahead - 1; ++k) request();
           // the lane's j: R_j, U'_j and -(1 - R_j^2) for the members a, and its tests here (all second
-          // members of the chunk, for each a, but j itself)
+          // members of the chunk, for each a, but j itself), taken off again where they are not run
           if (mine) {
             const int xj = 1 + it.slice + t_l * ns;  // block-local
             const float rij = ri[xj];
@@ -621,6 +626,7 @@ __device__ __forceinline__ void tests_l2_wide(const Launch &L, Wide2Smem &sm, Pe
               sm.s[wib][lane][a] = make_float4(R, (rij - ria[a] * R) * inv_i[a], R * R - 1.0f, 0.f);
               if (xa < d && xa != xj && hi >= lo) cnt += hi - lo + 1 - (xj >= lo && xj <= hi ? 1 : 0);
             }
+            sm.s[wib][lane][0].w = __int_as_float(cnt);
             executed += (unsigned)cnt;
           }
           __syncwarp();
@@ -632,7 +638,10 @@ __device__ __forceinline__ void tests_l2_wide(const Launch &L, Wide2Smem &sm, Pe
             const float4 v = sm.ring[wib][slot][lane];  // the lane's own copy
             slot = (slot + 1) & (kW2Ahead - 1);
             // removed by another warp meanwhile?
-            if (!((__shfl_sync(0xffffffffu, *(volatile unsigned *)&ls.alive[grp], 0) >> q) & 1u)) continue;
+            if (!((__shfl_sync(0xffffffffu, *(volatile unsigned *)&ls.alive[grp], 0) >> q) & 1u)) {
+              if (lane == q) executed -= (unsigned)__float_as_int(sm.s[wib][lane][0].w);
+              continue;
+            }
             const f32x2 r01 = pack2(-v.x, -v.y), r23 = pack2(-v.z, -v.w);  // -r_jb
             float low = 0.f, high = -1.f;
 #pragma unroll
@@ -678,13 +687,13 @@ __device__ __forceinline__ void tests_l2_wide(const Launch &L, Wide2Smem &sm, Pe
           __syncwarp();                                          // ... and so are the scalars
         }
       }
+      executed = __reduce_add_sync(0xffffffffu, executed);
+      if (lane == 0) atomicAdd(&ls.executed, (unsigned long long)executed);
     }
-    const unsigned long long ex = warp_sum_u64(executed);
     const unsigned rt = __reduce_add_sync(0xffffffffu, retests);
-    if (lane == 0) {
-      if (ex) atomicAdd(&I.ctr[2].tests, ex);
-      if (rt) atomicAdd(&I.ctr[2].retests, (unsigned long long)rt);
-    }
+    if (lane == 0 && rt) atomicAdd(&I.ctr[2].retests, (unsigned long long)rt);
+    __syncthreads();
+    if (tid == 0 && ls.executed) atomicAdd(&I.ctr[2].tests, ls.executed);
   }
   __syncwarp();
   flush_pending<2>(L, 2, pend, np);

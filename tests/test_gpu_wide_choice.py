@@ -85,3 +85,21 @@ def test_no_level_2_buffers_below_level_2():
         live.append(L.hpc_debug_live_allocations() - base)
         sk.close()
     assert live[1] == live[0] + 1  # level 1's snapshot
+
+
+def test_executed_tests_are_those_run():
+    """Every test of level 2 removes its edge, so an edge end is run by the warp that comes to it first
+    (seldom by a second one at the same time): about an eighth of the tests of a row's eight warps, not
+    those of every warp that once found it live."""
+    p = 64
+    sk = _context(p, 2)
+    _set_wide(sk, 1, 1)
+    sk.run()
+    for _ in range(3):
+        sk.reset()
+        st = sk.run()[2]
+        assert st["edges_before"] == p * (p - 1) // 2 and st["edges_after"] == 0
+        d = p - 1
+        per_warp = sum(d - a for a in range(1, 33)) / 8  # a warp's tests of one edge end, on average
+        assert 0 < st["executed_tests"] <= 2 * per_warp * p * d
+    sk.close()
