@@ -499,13 +499,14 @@ hpc_status global_errors(hpc_ctx *c) {
 }
 
 // A run to repeat from level 0: the neighbour lists were too small (the data changed
-// since they were sized), or the set order found the re-test queue full (the rerun
-// keeps the edge order, whose tests re-test inline when the queue is full).
+// since they were sized), or a queue-only kernel found the re-test queue full (the rerun
+// keeps the edge order, whose tests re-test inline when the queue is full; beside an FP64
+// matrix, in mixed precision, choose_defer1 sees the count).
 bool needs_rerun(hpc_ctx *c) {
   bool again = false;
   for (int b = 0; b < c->count; ++b) {
     const int err = c->gctr_host[b].err;
-    if (err & kErrRetestOverflow) c->set_off = true;
+    if ((err & kErrRetestOverflow) && c->opts.precision != HPC_PREC_MIXED) c->set_off = true;
     if (err & (kErrCsrOverflow | kErrRetestOverflow)) again = true;
   }
   return again;
@@ -616,8 +617,9 @@ hpc_status choose_wide(hpc_ctx *c, int last) {
 // a kernel of their own instead of re-testing inline: the inline FP64 re-test costs the
 // interleaved kernel registers (it spills) and a warp stops for its one lane. It takes a launch
 // more, so from kDefer1Tests potential tests (about edges2^2 / p) on; measured (p = 2000, 1.3e7 of
-// them): 129 us inline, 92 + 10 us with the kernel after it. A queue that overflows is rerun inline
-// (set_off), as in tensor-core mode.
+// them): 129 us inline, 92 + 10 us with the kernel after it. Where the context's last run re-tested more
+// than half a queue (a wide margin, ill-conditioned data) it stays inline; a queue that overflows all the
+// same is rerun once, inline by that count.
 constexpr double kDefer1Tests = 4e6;
 void choose_defer1(hpc_ctx *c) {
   c->defer1 = false;
@@ -625,15 +627,16 @@ void choose_defer1(hpc_ctx *c) {
       set_order_from() == 0)
     return;
   double tests = 0.0;
-  long long p2 = 0;
+  long long p2 = 0, retests = 0;
   for (int b = 0; b < c->count; ++b) {
     const double e2 = (double)c->ctr_host[(size_t)b * kLevels].edges2;
     tests += e2 * e2 / (double)c->ih[b].p;
     p2 += c->ih[b].p * c->ih[b].p;
+    retests += (long long)c->ctr_host[(size_t)b * kLevels + 1].retests;
   }
-  if (tests < kDefer1Tests) return;
+  const long long cap = c->rq ? c->rq_cap : std::min<long long>(1ll << 20, std::max<long long>(1ll << 14, p2 / 16));
+  if (tests < kDefer1Tests || 2 * retests > cap) return;
   if (!c->rq) {
-    const long long cap = std::min<long long>(1ll << 20, std::max<long long>(1ll << 14, p2 / 16));
     if (dev_alloc(&c->rq, cap, "re-test queue") != HPC_OK) return;  // re-tests inline, then
     c->rq_cap = cap;
     ++c->inst_version;  // a captured graph holds the queue pointer
