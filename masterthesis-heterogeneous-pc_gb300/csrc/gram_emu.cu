@@ -10,23 +10,31 @@
 //   y_v = sum_{t=1..7} d_t(v) 2^-7t     (d_1 = rint(128 y), then the remainders 7 bits
 //                                        at a time: integers, |d_1| <= 128, |d_t| <= 64,
 //                                        all exact in BF16; 49 bits of y)
-//   sum_k y_a y_b = sum_{t+u<=8} 2^-7(t+u) sum_k d_t(a) d_u(b)   (dropped pairs < 2^-56)
+//   sum_k y_a y_b = sum_{t+u<=8} 2^-7(t+u) sum_k d_t(a) d_u(b)   (weights below 2^-56 dropped)
 //
 // Each digit product is an integer of at most 2^14, so sums of a few hundred samples over
 // all the pairs (t, u) of one weight s = t + u are integers of at most 2^24: exact in the
 // tensor core's FP32 accumulator. The kernel keeps one TMEM accumulator per weight and runs
 // a block of 32 samples' digits against each other while they stand in shared memory: 56
 // MMAs for 112 KB of operands, where a pair at a time needs 28 times 16 KB. Seven 128-column
-// accumulators exceed the 512 columns of TMEM, so the samples go by twice: first the weights 2..5
-// (digits 1..4: 10 pairs), then 6..8 (all digits: 18 pairs). Every kGroupStages stages the
-// drain warps add the exact sums into 64-bit fixed-point integers (LSB 2^-47 of sum y_a y_b)
-// with integer instructions -- the FP64 pipe would be the bottleneck -- one weight after the
-// other, while the MMAs of the others go on. Where there are fewer tiles than SMs a cluster of
-// blocks shares a tile's samples and adds up the integers through distributed shared memory:
-// the result does not depend on the split. The epilogue scales by 2^(e_a + e_b) / (n - 1) and
-// writes the FP64 entry (both triangles) and its FP32 rounding. Error: the 49-bit digits and
-// the 2^-47 fixed point give |error| below 1e-13 on the correlation for n <= 32768 (the fixed
-// point's range bounds n).
+// accumulators exceed the 512 columns of TMEM, so the samples go by twice: first the weights 6..8
+// (all digits: 18 pairs), then 2..5 (digits 1..4: 10 pairs). Every kGroupStages stages the
+// drain warps add the exact sums into 64-bit fixed-point integers with integer instructions --
+// the FP64 pipe would be the bottleneck -- one weight after the other, while the MMAs of the
+// others go on. The first pass's integers have an LSB of 2^-56 of sum y_a y_b, which every weight
+// is a multiple of; between the passes they become an LSB of 2^-47 (the range of the whole sum for
+// n <= 32768) and the kLowBits below it. Where there are fewer tiles than SMs a cluster of blocks
+// shares a tile's samples; it adds up both through distributed shared memory and rounds once, as
+// a block alone does: the result does not depend on the split. The epilogue scales by
+// 2^(e_a + e_b) / (n - 1) and writes the FP64 entry (both triangles) and its FP32 rounding.
+//
+// Error of an entry, beside the roundings of FP64: the digits' 49 bits, at most 2^-50 (2^e_a +
+// 2^e_b); the dropped pairs, at most 6 * 2^12 * 2^-63 (1 + 2^-6) a sample, 2^(e_a + e_b - 48.3); the
+// rounding, 2^(e_a + e_b - 48) / (n - 1). 2^e is 8 for Gaussian data and at most 2 sqrt(n - 1), where one
+// sample outweighs all others. The dropped pairs' signs vary, so that they add up to far less:
+// measured against 113 bits, p = 257..2000, n = 2000..32768, the largest error is 1.2e-15 on Gaussian
+// data and 3.8e-13 where one sample of each variable is a thousand times the others (2.6e-15 and
+// 1.4e-12 with every group's sums of the weights 7 and 8 rounded down to 2^-47).
 //
 // Structure (one CTA of 10 warps per tile and part): warp 0 lane 0 TMA producer, warp 1 lane 0
 // MMA issuer (tcgen05.mma.kind::f16, M = N = 128, K = 16), warps 2-9 drain (TMEM lane quadrant
@@ -36,8 +44,9 @@
 //
 // Bound: the tensor cores and, beside them, the shared memory they read the operands from
 // (64 of every 80 cycles). Measured (this kernel): p = 2000, n = 5000 918 us with a pair at a
-// time, 497 us now (6.4e11 flops: 1.3 PFLOP/s); p = 1203, n = 3777, on 55 of 152 SMs then, 746 -> 207 us.
-// The digits 616 -> 53 us and 317 -> 27 us.
+// time, 462 us now (6.4e11 flops: 1.4 PFLOP/s; 497 us with a drain that shifts both ways, which the
+// first pass's LSB saves); p = 1203, n = 3777, on 55 of 152 SMs then, 746 -> 193 us. The digits
+// 616 -> 53 us and 317 -> 27 us.
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -56,12 +65,13 @@ namespace {
 constexpr int EM = 128, EN = 128, EK = 32;   // tile 128 x 128, 32 samples (64 B of a digit) per stage
 constexpr int kDigits = 7;
 constexpr int kTileBytes = EM * EK * 2;      // one digit's 128 rows of a stage: 8 KB
-// The two passes: weights s = 2..5 and 6..8 (accumulators 0..3 and 0..2), the digits they
-// need, and their stages -- both cut the same 224 KB.
-constexpr int kDigitsA = 4, kSlotsA = 4, kStagesA = 3, kBytesA = 2 * kDigitsA * kTileBytes;
-constexpr int kDigitsB = 7, kSlotsB = 3, kStagesB = 2, kBytesB = 2 * kDigitsB * kTileBytes;
-constexpr int kOperandBytes = kStagesB * kBytesB;
-static_assert(kStagesA * kBytesA <= kOperandBytes, "both passes share the operand buffer");
+// The two passes: weights s = 6..8 and 2..5 (accumulators 0..2 and 0..3), the digits they
+// need, and their stages -- both cut the same 224 KB, of which the second leaves 32 KB: there a
+// block of a cluster keeps its sums' low bits meanwhile.
+constexpr int kDigitsA = 7, kSlotsA = 3, kStagesA = 2, kBytesA = 2 * kDigitsA * kTileBytes;
+constexpr int kDigitsB = 4, kSlotsB = 4, kStagesB = 3, kBytesB = 2 * kDigitsB * kTileBytes;
+constexpr int kFirstA = 6, kFirstB = 2;  // their lowest weights
+constexpr int kOperandBytes = kStagesA * kBytesA;
 // Stages between two drains: the largest weight's sum grows by (2 * 2^13 + 5 * 2^12) a sample at
 // most (d_1 against d_7 twice, |d_1| <= 128, and five pairs of |d| <= 64), so 448 samples
 // stay below 2^24
@@ -71,19 +81,23 @@ constexpr int kTmemColsE = 512;              // four 128-column accumulators
 constexpr int kAccWarpsE = 8;
 constexpr int kThreadsE = 64 + 32 * kAccWarpsE;
 constexpr int kFixL = 47;                    // fixed-point LSB 2^-47
+constexpr int kLowBits = 9;                  // ... and the first pass's 2^-56
 constexpr int kMaxSplitE = 8;                // portable cluster size
 
 struct alignas(1024) EmuSmem {
   uint8_t operands[kOperandBytes];  // the stages; at the end a block's 128 x 128 integer sums
   uint64_t full_a[kStagesA], empty_a[kStagesA];
   uint64_t full_b[kStagesB], empty_b[kStagesB];
-  uint64_t acc_full[kSlotsA], acc_empty[kSlotsA];
+  uint64_t acc_full[kSlotsB], acc_empty[kSlotsB];
   uint64_t drain;
   uint32_t tmem_base;
   int abort;
 };
 static_assert(sizeof(EmuSmem) + 1024 <= 227 * 1024, "shared memory of a block");
-static_assert(sizeof(long long) * EM * EN <= kOperandBytes, "the sums fit the operand buffer");
+constexpr int kLowAt = kStagesB * kBytesB;   // the low bits, [column][row]
+static_assert(kLowAt + sizeof(uint16_t) * EM * EN <= kOperandBytes, "beside the second pass's stages");
+static_assert(sizeof(long long) * EM * EN <= kLowAt, "the sums fit before them");
+static_assert(kFixL + kLowBits == 7 * 8, "no bit of the lowest weight is lost");
 
 __device__ __forceinline__ bool aborted(EmuSmem &sm) { return *(volatile int *)&sm.abort != 0; }
 __device__ __forceinline__ void fail(EmuSmem &sm, int *err) {
@@ -186,7 +200,7 @@ __global__ void __launch_bounds__(kThreadsE, 1)
       mbar_init(&sm.full_b[s], 1);
       mbar_init(&sm.empty_b[s], 1);
     }
-    for (int c = 0; c < kSlotsA; ++c) {
+    for (int c = 0; c < kSlotsB; ++c) {
       mbar_init(&sm.acc_full[c], 1);
       mbar_init(&sm.acc_empty[c], kAccWarpsE);
     }
@@ -245,7 +259,7 @@ __global__ void __launch_bounds__(kThreadsE, 1)
   } else if (warp == 1 && lane == 0) {
     // MMA issuer. Pass P: accumulator c takes the digit pairs of weight first + c; a stage's MMAs of
     // one accumulator after the other, so that a drained one is refilled while the next is drained.
-    // fill: how often the accumulators were filled before (their barriers' phases)
+    // fill: how often the first kSlotsA accumulators were filled before (their barriers' phases)
     auto run = [&](int first, int slots, int digits, int nstages, int bytes, uint64_t *full, uint64_t *empty,
                    int fill) {
       for (int k = 0; k < nk && !aborted(sm); ++k) {
@@ -258,8 +272,9 @@ __global__ void __launch_bounds__(kThreadsE, 1)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a0 = smem_u32(sm.operands + s * bytes), b0 = a0 + digits * kTileBytes;
         for (int c = 0; c < slots; ++c) {
-          if (begin && fill + g > 0) {
-            if (!mbar_wait(&sm.acc_empty[c], (fill + g - 1) & 1)) {
+          const int before = (c < kSlotsA ? fill : 0) + g;
+          if (begin && before > 0) {
+            if (!mbar_wait(&sm.acc_empty[c], (before - 1) & 1)) {
               fail(sm, err);
               break;
             }
@@ -278,8 +293,8 @@ __global__ void __launch_bounds__(kThreadsE, 1)
         mma_commit(&empty[s]);
       }
     };
-    run(2, kSlotsA, kDigitsA, kStagesA, kBytesA, sm.full_a, sm.empty_a, 0);
-    run(2 + kSlotsA, kSlotsB, kDigitsB, kStagesB, kBytesB, sm.full_b, sm.empty_b, groups);
+    run(kFirstA, kSlotsA, kDigitsA, kStagesA, kBytesA, sm.full_a, sm.empty_a, 0);
+    run(kFirstB, kSlotsB, kDigitsB, kStagesB, kBytesB, sm.full_b, sm.empty_b, groups);
     mma_commit(&sm.drain);
     if (!mbar_wait(&sm.drain, 0)) fail(sm, err);
   } else if (warp >= 2) {
@@ -289,17 +304,18 @@ __global__ void __launch_bounds__(kThreadsE, 1)
 #pragma unroll
     for (int q = 0; q < kCols; ++q) acc[q] = 0;
     for (int pass = 0; pass < 2 && ok; ++pass) {
-      const int slots = pass ? kSlotsB : kSlotsA, first = pass ? 2 + kSlotsA : 2;
+      const int slots = pass ? kSlotsB : kSlotsA, first = pass ? kFirstB : kFirstA;
+      const int lsb = pass ? kFixL : kFixL + kLowBits;
       for (int g = 0; g < groups && ok; ++g)
         for (int c = 0; c < slots; ++c) {
-          if (!mbar_wait(&sm.acc_full[c], (pass * groups + g) & 1)) {
+          if (!mbar_wait(&sm.acc_full[c], ((pass && c < kSlotsA ? groups : 0) + g) & 1)) {
             fail(sm, err);
             ok = false;
             break;
           }
           __syncwarp();
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const int sh = kFixL - 7 * (first + c);  // the sum's weight 2^-7s in units of 2^-47
+          const int sh = lsb - 7 * (first + c);  // the sum's weight 2^-7s in units of 2^-lsb
 #pragma unroll
           for (int c0 = 0; c0 < kCols; c0 += 16) {
             float v[16];
@@ -307,13 +323,24 @@ __global__ void __launch_bounds__(kThreadsE, 1)
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
               const long long gi = (long long)__float2int_rn(v[q]);  // an integer of at most 2^24: exact
-              acc[c0 + q] += sh >= 0 ? (long long)((unsigned long long)gi << sh) : (gi >> (-sh));
+              acc[c0 + q] += (long long)((unsigned long long)gi << sh);
             }
           }
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) mbar_arrive(&sm.acc_empty[c]);
         }
+      if (pass == 0 && ok) {
+        // to the LSB of the whole sum: rounded, or with the low bits kept for the cluster's sum (the first
+        // pass's MMAs have all completed, and the second's copies end before kLowAt)
+        uint16_t *low = reinterpret_cast<uint16_t *>(sm.operands + kLowAt) + half * kCols * EM + quad * 32 + lane;
+#pragma unroll
+        for (int q = 0; q < kCols; ++q) {
+          if (split > 1) low[q * EM] = (uint16_t)(acc[q] & ((1 << kLowBits) - 1));
+          else acc[q] += 1 << (kLowBits - 1);
+          acc[q] >>= kLowBits;
+        }
+      }
     }
   }
   __syncwarp();
@@ -342,7 +369,7 @@ __global__ void __launch_bounds__(kThreadsE, 1)
     }
   } else {
     // the parts' sums: each block keeps its own in its operand buffer (every copy and MMA has
-    // completed), then adds up and writes its share of the columns
+    // completed; the low bits stand behind), then adds up and writes its share of the columns
     cg::cluster_group cluster = cg::this_cluster();
     long long *sums = reinterpret_cast<long long *>(sm.operands);  // [column][row]
     __syncthreads();
@@ -357,8 +384,12 @@ __global__ void __launch_bounds__(kThreadsE, 1)
       const int lo = EN * part / split, hi = EN * (part + 1) / split;
       for (int cc = lo + ((warp - 2) >> 2); cc < hi; cc += 2) {
         long long sum = 0;
-        for (int q = 0; q < split; ++q) sum += cluster.map_shared_rank(sums, q)[cc * EM + r];
-        write(row, (int64_t)bj * EN + cc, sum, er);
+        int low = 1 << (kLowBits - 1);
+        for (int q = 0; q < split; ++q) {
+          sum += cluster.map_shared_rank(sums, q)[cc * EM + r];
+          low += cluster.map_shared_rank(reinterpret_cast<uint16_t *>(sm.operands + kLowAt), q)[cc * EM + r];
+        }
+        write(row, (int64_t)bj * EN + cc, sum + (low >> kLowBits), er);
       }
     }
     cluster.sync();  // no block leaves while its sums are read
