@@ -124,10 +124,16 @@ hpc_status hpc_ctx_set_stream(hpc_ctx *ctx, void *stream);
 hpc_status hpc_ctx_set_graphs(hpc_ctx *ctx, int enable);
 /* Device-time breakdown of the context's last correlation and levels. */
 hpc_status hpc_get_timings(hpc_ctx *ctx, hpc_timings *out);
-/* Device bytes held by a context of this shape (admission control). Dense graphs take more,
- * as they come: neighbour lists and records for their edges, and up to about 6 MB a thread block
- * (two blocks an SM) for levels 1 and 2 on wide rows, which run without where there is no room. */
+/* Device bytes held by a context of this shape (admission control). Dense graphs take more, as
+ * they come: neighbour lists and records for their edges, and the buffers of hpc_ctx_footprint_wide. */
 hpc_status hpc_ctx_footprint(int64_t p, int64_t n_obs, const hpc_opts *opts, int64_t *bytes);
+/* Device bytes that such a context may take beside hpc_ctx_footprint for levels 1 and 2 of dense
+ * data in the mixed modes, and then keeps: a copy of the adjacency bits (level 1 on wide rows), a queue of
+ * rows and, for each of two blocks an SM, max(2^20, 32 p) + 33 p floats (level 2 on wide rows: 1.4 GB at
+ * p = 2000, 1.6 GB at 9000, 4.5 GB at 46340), and a queue of at most 151 MB (level 1's re-tests beside an
+ * FP64 matrix). 0 where none can come to use. A level without room for its part runs without it; the
+ * server's requests take none. A batch takes the level-2 part of its largest problem. */
+hpc_status hpc_ctx_footprint_wide(int64_t p, const hpc_opts *opts, int64_t *bytes);
 
 /* ---- correlation --------------------------------------------------------
  * Replaces gpuPMCC(h_mat, n, dim, cors, deviceId, verbose)

@@ -564,6 +564,7 @@ hpc_status sync_tune(hpc_ctx *c) {
 // context's life; the other level does not depend on it.
 constexpr long long kWide2Rows = 1500;
 constexpr double kWide2Deg = 40.0;
+constexpr int64_t kWide2Blocks = 2 * 152;  // most blocks of level 2's kernel: two an SM
 hpc_status choose_wide(hpc_ctx *c, int last) {
   c->wide1 = c->wide2 = false;
   if (c->opts.precision == HPC_PREC_FP64) return HPC_OK;
@@ -621,6 +622,7 @@ hpc_status choose_wide(hpc_ctx *c, int last) {
 // than half a queue (a wide margin, ill-conditioned data) it stays inline; a queue that overflows all the
 // same is rerun once, inline by that count.
 constexpr double kDefer1Tests = 4e6;
+long long defer1_cap(long long p2) { return std::min<long long>(1ll << 20, std::max<long long>(1ll << 14, p2 / 16)); }
 void choose_defer1(hpc_ctx *c) {
   c->defer1 = false;
   if (c->opts.precision != HPC_PREC_MIXED || !c->cor64_valid || c->set_off || c->level_by_level || !c->level0_known ||
@@ -634,7 +636,7 @@ void choose_defer1(hpc_ctx *c) {
     p2 += c->ih[b].p * c->ih[b].p;
     retests += (long long)c->ctr_host[(size_t)b * kLevels + 1].retests;
   }
-  const long long cap = c->rq ? c->rq_cap : std::min<long long>(1ll << 20, std::max<long long>(1ll << 14, p2 / 16));
+  const long long cap = c->rq ? c->rq_cap : defer1_cap(p2);
   if (tests < kDefer1Tests || 2 * retests > cap) return;
   if (!c->rq) {
     if (dev_alloc(&c->rq, cap, "re-test queue") != HPC_OK) return;  // re-tests inline, then
@@ -1116,6 +1118,21 @@ hpc_status hpc_ctx_footprint(int64_t p, int64_t n, const hpc_opts *o, int64_t *b
     b += cap * ((int64_t)sizeof(RetestItem) + 4) + retest_scratch_entries(cap) * 8;  // queue, counters, entries
   }
   *bytes = b;
+  return HPC_OK;
+}
+
+hpc_status hpc_ctx_footprint_wide(int64_t p, const hpc_opts *o, int64_t *bytes) {
+  if (!o || !bytes || p < 2) return HPC_ERR_INVALID_ARG;
+  *bytes = 0;
+  if (o->precision == HPC_PREC_FP64 || o->max_level == 0) return HPC_OK;
+  const WideShape complete{p, p * (p - 1)};
+  const bool wide1 = wide1_pays(&complete, 1);
+  if (wide1) *bytes += p * ((p + 31) / 32) * 4;  // adj0
+  if (o->max_level != 1 && (wide1 || p >= kWide2Rows))
+    *bytes += p * (int64_t)wide2_slices(p - 1, p) * (int64_t)sizeof(WideItem) +
+              kWide2Blocks * wide2_floats(p - 1) * (int64_t)sizeof(float);
+  if (o->precision == HPC_PREC_MIXED && (double)p * (double)(p - 1) * (double)(p - 1) >= kDefer1Tests)
+    *bytes += defer1_cap(p * p) * (int64_t)sizeof(RetestItem);
   return HPC_OK;
 }
 

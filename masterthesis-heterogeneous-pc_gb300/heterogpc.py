@@ -95,6 +95,7 @@ _SIGS = {
     "hpc_ctx_destroy": (C.c_int, [C.c_void_p]),
     "hpc_ctx_reset": (C.c_int, [C.c_void_p]),
     "hpc_ctx_footprint": (C.c_int, [C.c_int64, C.c_int64, C.POINTER(Opts), C.POINTER(C.c_int64)]),
+    "hpc_ctx_footprint_wide": (C.c_int, [C.c_int64, C.POINTER(Opts), C.POINTER(C.c_int64)]),
     "hpc_ctx_set_stream": (C.c_int, [C.c_void_p, C.c_void_p]),
     "hpc_get_timings": (C.c_int, [C.c_void_p, C.POINTER(Timings)]),
     "hpc_ctx_set_graphs": (C.c_int, [C.c_void_p, C.c_int]),
