@@ -136,12 +136,13 @@ constexpr int64_t kW2Floats = 1 << 20;  // copied entries of a slice, about
 // leading dimension of the copied block of a row of degree d: the row itself and its neighbours,
 // rows of whole 16-byte words
 __host__ __device__ __forceinline__ int64_t wide2_ld(int64_t d) { return (d + 1 + 3) & ~(int64_t)3; }
-// A row is split where its slice would not fit the scratch, and below p = 6000 also at 256
-// neighbours: there are too few rows then to keep every block busy beside its widest ones
-// (p = 3001: 5.2 -> 3.0 ms), while with more rows the copies of the rows beside the slices cost
-// more than they save (p = 9000: 79 -> 48 ms without).
+// A row is split where its slice would not fit the scratch, and below p = 7000 also at 256
+// neighbours: there are too few rows then to keep every block busy beside its widest ones, while
+// with more rows the copies of the rows beside the slices cost more than they save. Level 2 with
+// slices of 256 and of 1024, preferential attachment, ms: p = 3001 3.2 / 4.6, 4500 9.2 / 11.4, 5500
+// 13.9 / 14.4, 6500 25.7 / 31.3, 7500 27.4 / 20.7, 9000 44.8 / 34.4, 12000 275 / 188, 15000 231 / 140.
 __host__ __device__ __forceinline__ int wide2_slice(int64_t d, int64_t p) {
-  const int64_t s = kW2Floats / wide2_ld(d), most = p < 6000 ? 256 : kW2Slice;
+  const int64_t s = kW2Floats / wide2_ld(d), most = p < 7000 ? 256 : kW2Slice;
   return (int)(s < 32 ? 32 : s > most ? most : s);
 }
 __host__ __device__ __forceinline__ int wide2_slices(int64_t d, int64_t p) {
