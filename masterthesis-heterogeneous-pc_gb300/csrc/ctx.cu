@@ -617,11 +617,12 @@ hpc_status choose_wide(hpc_ctx *c, int last) {
 // Whether level 1 of a context with an FP64 matrix (mixed precision) queues its undecided tests for
 // a kernel of their own instead of re-testing inline: the inline FP64 re-test costs the
 // interleaved kernel registers (it spills) and a warp stops for its one lane. It takes a launch
-// more, so from kDefer1Tests potential tests (about edges2^2 / p) on; measured (p = 2000, 1.3e7 of
-// them): 129 us inline, 92 + 10 us with the kernel after it. Where the context's last run re-tested more
+// more, so from kDefer1Tests potential tests (about edges2^2 / p) on. Levels 0 and 1 inline / queued, us:
+// 1.4e6 tests (p = 700) 101 / 102, 2.6e6 (1000) 126 / 115, 4.3e6 (1300) 152 / 139, 9.2e6 (2000) 199 / 166; the
+// same within 1 % below 1e6. Where the context's last run re-tested more
 // than half a queue (a wide margin, ill-conditioned data) it stays inline; a queue that overflows all the
 // same is rerun once, inline by that count.
-constexpr double kDefer1Tests = 4e6;
+constexpr double kDefer1Tests = 2e6;
 long long defer1_cap(long long p2) { return std::min<long long>(1ll << 20, std::max<long long>(1ll << 14, p2 / 16)); }
 void choose_defer1(hpc_ctx *c) {
   c->defer1 = false;
