@@ -1281,6 +1281,7 @@ hpc_status hpc_autotune(hpc_ctx *c, const hpc_tune_params *cands, int ncands, in
   }
   const bool graphs = c->graphs_enabled;
   const TuneEntry force0 = c->tune_force;
+  const bool set_off0 = c->set_off;  // a candidate's kernels may fill the re-test queue where the context's do not
   c->graphs_enabled = false;  // kernel by kernel: every level's kernels are timed
   // every candidate's level times, the candidates taken in turn within each round (so
   // that a drift over the tuning run touches them alike); per level the candidate with
@@ -1321,6 +1322,7 @@ hpc_status hpc_autotune(hpc_ctx *c, const hpc_tune_params *cands, int ncands, in
     }
   }
   c->tune_force = force0;
+  c->set_off = set_off0;
   c->graphs_enabled = graphs;
   ++c->inst_version;
   const hpc_status reset = hpc_ctx_reset(c);

@@ -54,6 +54,28 @@ def test_autotune_times_the_kernels_that_read_the_policies(capfd):
     hg.tune_clear()
 
 
+def test_autotune_leaves_the_queue_in_use():
+    """The candidates' kernels run every re-test from both rows and overflow a queue that the wide level 1
+    does not fill: they are timed with it off, the context keeps it."""
+    p, n = 1200, 2000
+    rng = np.random.default_rng(9)
+    X = (rng.standard_normal((1, n)) + rng.standard_normal((p, n))).astype(np.float32)
+    hg.tune_clear()
+    sk = hg.SkeletonCalculator(p, n, alpha=0.05, max_level=1, precision=hg.PREC_MIXED_TC, retest_margin=4.5)
+    sk.add_observations(X)
+    assert _level1(sk) == 0.5
+    retests = sk.level_stats[1]["retests"]
+    assert retests > 100
+    assert hg.lib().hpc_debug_set_retest_queue(sk.handle, retests * 3 // 2) == 0
+    sk.autotune([{"tile_cap": 64, "tiles_per_lane": 4, "edge_lanes": 32, "l1_prefetch": 0}], reps=1)
+    assert hg.lib().hpc_debug_set_order_active(sk.handle) == 1
+    for _ in range(2):
+        assert _level1(sk) == 0.5 and sk.level_stats[1]["retests"] == retests
+    assert hg.lib().hpc_debug_set_order_active(sk.handle) == 1
+    sk.close()
+    hg.tune_clear()
+
+
 def test_no_room_for_level_2_leaves_level_1_alone():
     L = hg.lib()
     sk = _context(1600, 2)
