@@ -558,7 +558,8 @@ hpc_status sync_tune(hpc_ctx *c) {
 // run), level 2 by its degrees in the last run -- before a first run, where level 1 is wide.
 // Level 2 needs kWide2Rows rows of a mean degree of kWide2Deg to keep its blocks busy (measured,
 // ordinary against wide: mean degree 41 of 1000 rows 405 / 455 us, 35 of 700 248 / 508 us; 65 of 1500
-// 1794 / 966 us, 85 of 2000 4.9 / 2.3 ms, 51 of 2000 1.92 / 1.95 ms, 42 of 8000 7.0 / 2.1 ms). (The
+// 1794 / 966 us, 85 of 2000 4.9 / 2.3 ms, 51 of 2000 1.92 / 1.95 ms, 42 of 8000 7.0 / 2.1 ms, 364 of
+// 15000 2685 / 141 ms). (The
 // kernel of level 2 takes the wide rows and leaves the others to the ordinary body, so a wrong guess
 // costs time only.) A level without room for its buffers runs the ordinary kernel, for the rest of the
 // context's life; the other level does not depend on it.
@@ -1020,8 +1021,8 @@ bool uses_set_order(int set_from, int level) {
 // Level 1 on wide rows costs about 0.8 ns an edge (p up to 3000; 1.1 ns at 9000) and more where
 // the rows hold little of the p variables that it goes over, the ordinary body 2-4 ps an edge and
 // neighbour. Measured, ordinary against wide: mean degree 474 of p = 700 280 / 473 us, 638 of 1000
-// 550 / 503 us, 1029 of 1500 1773 / 634 us, 1645 of 3000 6411 / 1928 us; 444 of 8000 3415 / 4395 us,
-// 237 of 4000 538 / 911 us, a batch of 512 (p up to 800, 42) 3.2 / 3.7 ms. So from a mean degree of
+// 550 / 503 us, 1029 of 1500 1773 / 634 us, 1645 of 3000 6411 / 1928 us, 9324 of 15000 1592 / 98 ms; 444 of
+// 8000 3415 / 4395 us, 237 of 4000 538 / 911 us, a batch of 512 (p up to 800, 42) 3.2 / 3.7 ms. So from a mean degree of
 // kWide1Deg on, where that is an eighth of p or more and there are items for every SM.
 constexpr double kWide1Deg = 600.0, kWide1Density = 1.0 / 8.0;
 static double wide1_items(const WideShape *sh, int count, int cols) {
